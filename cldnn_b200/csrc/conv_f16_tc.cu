@@ -24,6 +24,7 @@
 #include <mutex>
 #include <string>
 #include "engine.hpp"
+#include "conv_featrows.hpp"
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -447,10 +448,12 @@ static bool f16_driver_entry_points()
     return h_encode_tiled && h_encode_im2col;
 }
 
-struct F16Plan { int a_mode, bn, bk, bw, bh, bb; };
+struct F16Plan { int a_mode, bn, bk, bw, bh, bb; bool featrows; FrPlan fr; };
 static const int kF16TuneBN[3] = {64, 128, 256};
 // tune index -> (addressing mode, feature tile): 1 + mode * 3 + {64, 128, 256}; 0 = automatic
-static int f16_tune_count(const void*) { return 1 + 4 * 3; }           // 1 + 3 * mode + feature tile; modes flat / im2col / tiled / patch
+// 1 + 3 * mode + feature tile; modes flat / im2col / tiled / patch; 13..32: the feature-row form (conv_featrows.cu)
+constexpr int kF16TuneFeatRows = 13;
+static int f16_tune_count(const void*) { return kF16TuneFeatRows + kFrVariants; }
 constexpr size_t kF16PatchWeightBytes = 80 * 1024;                  // largest weight tensor the patch mode keeps resident
 
 static bool f16_dense(const cldnn_b200_tensor& t) { return t.py == t.px * t.x && t.pb == t.py * t.y; }
@@ -513,6 +516,12 @@ static bool f16_plan(const cldnn_b200_conv_params& p, F16Plan& pl, std::string* 
     const bool im2col_ok = p.pad_x <= 127 && p.pad_y <= 127 && (p.kw - 1) * p.dil_x <= 255 && (p.kh - 1) * p.dil_y <= 255 &&
                            p.stride_x <= 8 && p.stride_y <= 8 && (int64_t)p.in.b * p.in.pb * 2 >= 131072;
     int mode = -1, bn = 0;
+    pl.featrows = false;
+    if (p.tune == 0) {
+        const int v = fr_inner_product_variant(p);
+        if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
+    }
+    if (p.tune >= kF16TuneFeatRows) { pl.featrows = true; return fr_plan(p, p.tune - kF16TuneFeatRows, pl.fr, why); }
     if (p.tune > 0) { mode = (p.tune - 1) / 3; bn = kF16TuneBN[(p.tune - 1) % 3]; }
     if (mode < 0) mode = is_1x1_s1 ? f16tc::A_FLAT : (im2col_ok ? f16tc::A_IM2COL : f16tc::A_TILED);
     if (mode == f16tc::A_FLAT && !is_1x1_s1) return no("flat addressing needs a dense 1x1 stride-1 convolution");
@@ -596,6 +605,7 @@ static int32_t f16_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn
         return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: buffers must be 16-byte aligned");
     if (!f16_driver_entry_points()) return fail(CLDNN_B200_DEVICE_ERROR, "conv_f16_tc: the CUDA driver does not export cuTensorMapEncodeTiled/Im2col");
 
+    if (pl.featrows) return fr_prepare(ctx, p, a, pl.fr, out);
     Params P{};
     P.a_mode = pl.a_mode;
     P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;

@@ -25,6 +25,7 @@
 #include <cuda.h>
 #include <mutex>
 #include "conv_i8_tc.hpp"
+#include "conv_featrows.hpp"
 #include "conv_epilogue.cuh"
 
 namespace b200 {
@@ -385,7 +386,7 @@ static bool load_driver_entry_points()
     return g_encode_tiled && g_encode_im2col;
 }
 
-struct TcPlan { int a_mode; int bn; int bk; int bw, bh, bb; int epi_groups; int pair; };
+struct TcPlan { int a_mode; int bn; int bk; int bw, bh, bb; int epi_groups; int pair; bool featrows; FrPlan fr; };
 
 // tune index -> (addressing mode, feature tile).  0 = automatic choice.
 static const int kTuneBN[4] = {32, 64, 128, 256};
@@ -395,8 +396,10 @@ static const int kTuneBN[4] = {32, 64, 128, 256};
 // (16 epilogue warps per SM: for the layers whose time is the epilogue's instruction issue).
 // 45..50: CTA pairs on the specialised kernel (two epilogue groups): 45 + 2 * mode + {128, 256}[i], mode flat / im2col / tiled
 constexpr int kTuneFourGroups = 28;
+// 51..70: the feature-row form (conv_featrows.cu)
 constexpr int kTunePair = 44;
-static int tc_tune_count(const void*) { return 1 + 2 * 3 * 4 + 4 + 3 * 4 + 4 + 6; }
+constexpr int kTuneFeatRows = 51;
+static int tc_tune_count(const void*) { return kTuneFeatRows + kFrVariants; }
 constexpr size_t kPatchWeightBytes = 72 * 1024;       // largest weight tensor the patch mode keeps resident
 
 static bool dense_byxf(const cldnn_b200_tensor& t)
@@ -495,7 +498,12 @@ static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* wh
                            (int64_t)p.in.b * p.in.pb >= 131072;     // small tensors take the tiled path
     int tune = p.tune;
     int mode = -1, bn = 0;
-    pl.epi_groups = 2; pl.pair = 0;
+    pl.epi_groups = 2; pl.pair = 0; pl.featrows = false;
+    if (tune == 0) {
+        const int v = fr_inner_product_variant(p);
+        if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
+    }
+    if (tune >= kTuneFeatRows) { pl.featrows = true; return fr_plan(p, tune - kTuneFeatRows, pl.fr, why); }
     if (tune > kTunePair) {
         if (tune > kTunePair + 6) return no("unknown tuning index");
         if (!lean_params(p)) return no("CTA pairs exist on the specialised kernel only");
@@ -589,6 +597,7 @@ static int32_t tc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_
     if (((uintptr_t)a->input0 | (uintptr_t)a->weights) & 15) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: input and weights must be 16-byte aligned");
     if (!load_driver_entry_points()) return fail(CLDNN_B200_DEVICE_ERROR, "conv_i8_tc: the CUDA driver does not export cuTensorMapEncodeTiled/Im2col");
 
+    if (pl.featrows) return fr_prepare(ctx, p, a, pl.fr, out);
     TcParams P{};
     P.a_mode = pl.a_mode;
     P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;

@@ -59,8 +59,6 @@ struct FastAux {
 size_t tc_fast_aux_bytes() { return sizeof(FastAux); }
 
 
-__device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A K-major swizzled operand descriptor split in halves: the high word is constant per launch
 // (8-row group stride, descriptor version, swizzle mode), the low word holds the start address.
 __device__ __forceinline__ uint32_t desc_hi(uint32_t sbo_bytes, uint32_t layout_type)

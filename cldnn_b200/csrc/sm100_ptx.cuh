@@ -86,6 +86,10 @@ __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, vo
     return mbar_wait_slow(bar, parity, s_abort, g_status, code);
 }
 
+// ---- programmatic dependent launch ------------------------------------------------
+__device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- TMA ---------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const void* tmap)
 {
