@@ -4,8 +4,23 @@
 // feature-innermost fast path with 16-byte accesses per lane.
 #include <cuda_fp16.h>
 #include "engine.hpp"
+#include "sm100_ptx.cuh"
 
 namespace b200 {
+
+// Launch with programmatic stream serialisation: the kernel's blocks may be scheduled while the previous kernel of the stream
+// drains, so it executes griddepcontrol.wait before it touches memory.
+template <class... Params, class... Args>
+static cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
 
 static inline int grid_for(int64_t total, int threads, const cldnn_b200_ctx_impl* ctx)
 {
@@ -777,12 +792,105 @@ reorder_ref_kernel(const __grid_constant__ cldnn_b200_reorder_params p, const vo
         store_sat_float(out, p.out.dtype, oi, v);
     }
 }
+// The same between a planar layout (bfyx) and a feature-innermost one (byxf) of equal element type, 1 or 2 bytes: per image a
+// transposition of features x pixels.  Walking the destination in order (the kernel above) reads one element per 32-byte sector
+// of the source: 32 x 512 x 28 x 28 halves (51 MB moved) took 95 us.  Here a block moves a tile of 64 features x 64 pixels through
+// shared memory, both sides in vectors along their contiguous axis: 16 bytes of features, VB bytes of pixels (16, 4 or one
+// element, whatever the planes' size keeps aligned).  13 - 18 us for the same tensor, 2.9 - 4.0 TB/s; tiles are small so that one
+// image still makes many blocks.
+// (No early release of dependents: weights are packed with this kernel, and convolutions fetch weights before they wait.)
+constexpr int kTileF = 64, kTileP = 64, kTilePitch = kTileP + 2;
+template <class T, int VB, bool kToByxf>
+__global__ void __launch_bounds__(256)
+reorder_tile_kernel(const T* __restrict__ in, T* __restrict__ out, int F, int Fs, int HW, int64_t plane_pf, int64_t plane_pb, int64_t inner_px, int64_t inner_pb)
+{
+    constexpr int VP = VB / (int)sizeof(T), VF = 16 / (int)sizeof(T);          // elements per vector: planar side, byxf side
+    __shared__ T tile[kTileF][kTilePitch];
+    ptx::griddep_wait();
+    const int f0 = blockIdx.x * kTileF, p0 = blockIdx.y * kTileP, b = blockIdx.z;
+    auto planar = [&](bool load) {
+        for (int i = threadIdx.x; i < kTileF * (kTileP / VP); i += 256) {
+            const int f = i / (kTileP / VP), p = (i - f * (kTileP / VP)) * VP;
+            if (p0 + p >= HW || (!load && f0 + f >= F)) continue;              // planes hold whole vectors
+            union { T e[VP]; uint4 q[(VB + 15) / 16]; uint32_t w[(VB + 3) / 4]; } v;
+            const int64_t at = b * plane_pb + (int64_t)(f0 + f) * plane_pf + p0 + p;
+            if (load) {
+                if (f0 + f >= F) { for (int k = 0; k < VP; ++k) v.e[k] = T(0); }
+                else if (VB == 16) v.q[0] = *reinterpret_cast<const uint4*>(in + at);
+                else if (VB == 4) v.w[0] = *reinterpret_cast<const uint32_t*>(in + at);
+                else v.e[0] = in[at];
+#pragma unroll
+                for (int k = 0; k < VP; ++k) tile[f][p + k] = v.e[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < VP; ++k) v.e[k] = tile[f][p + k];
+                if (VB == 16) *reinterpret_cast<uint4*>(out + at) = v.q[0];
+                else if (VB == 4) *reinterpret_cast<uint32_t*>(out + at) = v.w[0];
+                else out[at] = v.e[0];
+            }
+        }
+    };
+    auto inner = [&](bool load) {
+        for (int i = threadIdx.x; i < kTileP * (kTileF / VF); i += 256) {
+            const int p = i / (kTileF / VF), f = (i - p * (kTileF / VF)) * VF;
+            if (p0 + p >= HW || f0 + f >= Fs) continue;                        // the stored feature count is in whole vectors
+            union { T e[VF]; uint4 q; } v;
+            const int64_t at = b * inner_pb + (int64_t)(p0 + p) * inner_px + f0 + f;
+            if (load) {
+                v.q = *reinterpret_cast<const uint4*>(in + at);
+#pragma unroll
+                for (int k = 0; k < VF; ++k) tile[f + k][p] = v.e[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < VF; ++k) v.e[k] = tile[f + k][p];
+                *reinterpret_cast<uint4*>(out + at) = v.q;
+            }
+        }
+    };
+    if (kToByxf) planar(true); else inner(true);
+    __syncthreads();
+    if (kToByxf) inner(false); else planar(false);
+}
+
+template <class T, bool kToByxf>
+static std::function<cudaError_t(cudaStream_t)> reorder_tile_launch(int vb, dim3 grid, const void* in, void* out, int F, int Fs, int HW, int64_t ppf, int64_t ppb, int64_t ipx, int64_t ipb)
+{
+    auto* k = vb == 16 ? reorder_tile_kernel<T, 16, kToByxf> : (vb == 4 ? reorder_tile_kernel<T, 4, kToByxf> : reorder_tile_kernel<T, (int)sizeof(T), kToByxf>);
+    return [=](cudaStream_t s) { return launch_dependent(k, grid, 256, s, (const T*)in, (T*)out, F, Fs, HW, ppf, ppb, ipx, ipb); };
+}
+
+// the tile kernel's launch, or an empty function when the two layouts are not its pair
+static std::function<cudaError_t(cudaStream_t)> reorder_tile_form(const cldnn_b200_reorder_params& p, const void* in, void* out)
+{
+    const int es = dtype_bytes(p.in.dtype);
+    if (p.has_mean || p.in.dtype != p.out.dtype || (es != 1 && es != 2)) return {};
+    const bool to = p.in.px == 1 && p.out.pf == 1 && p.out.px > 1, from = p.in.pf == 1 && p.in.px > 1 && p.out.px == 1;
+    if (!to && !from) return {};
+    const cldnn_b200_tensor& pl = to ? p.in : p.out; const cldnn_b200_tensor& nn = to ? p.out : p.in;
+    const int64_t HW = (int64_t)pl.y * pl.x, Fs = to ? p.out.f : (p.in.f + 15) / 16 * 16, vf = 16 / es;
+    if (HW < 8 || pl.py != pl.x || nn.py != nn.px * nn.x || HW >= (1 << 30)) return {};
+    if (nn.px % vf || nn.pb % vf || nn.offset % vf || Fs % vf || Fs > nn.px || (!to && p.out.f != p.in.f)) return {};
+    const char* ia = (const char*)in + (int64_t)p.in.offset * es; char* oa = (char*)out + (int64_t)p.out.offset * es;
+    if ((uintptr_t)(to ? oa : ia) & 15) return {};
+    int vb = es;
+    for (int v : {16, 4}) if ((HW * es) % v == 0 && (pl.pf * es) % v == 0 && (pl.pb * es) % v == 0 && ((uintptr_t)(to ? ia : oa)) % v == 0) { vb = v; break; }
+    const dim3 grid((unsigned)((Fs + kTileF - 1) / kTileF), (unsigned)((HW + kTileP - 1) / kTileP), (unsigned)p.in.b);
+    if (grid.y > 65535u || grid.z > 65535u || grid.z == 0) return {};
+    const int F = p.in.f;
+    if (es == 1) return to ? reorder_tile_launch<uint8_t, true>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb)
+                           : reorder_tile_launch<uint8_t, false>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb);
+    return to ? reorder_tile_launch<uint16_t, true>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb)
+              : reorder_tile_launch<uint16_t, false>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb);
+}
+
 static bool reorder_supports(const void* vp) { const auto& p = *(const cldnn_b200_reorder_params*)vp; return p.in.b == p.out.b && p.in.y == p.out.y && p.in.x == p.out.x && p.out.f >= p.in.f; }
 static int32_t reorder_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)
 {
     const cldnn_b200_reorder_params p = *(const cldnn_b200_reorder_params*)vp;
     if (!a->input0 || !a->output) return fail(CLDNN_B200_INVALID_ARG, "reorder_ref: input and output are required");
     const void* in = a->input0; void* o = a->output;
+    out->fn = reorder_tile_form(p, in, o);
+    if (out->fn) return CLDNN_B200_SUCCESS;
     const int grid = grid_for((int64_t)p.out.b * p.out.f * p.out.y * p.out.x, 256, ctx);
     out->fn = [=](cudaStream_t s) { reorder_ref_kernel<<<grid, 256, 0, s>>>(p, in, o); return cudaGetLastError(); };
     return CLDNN_B200_SUCCESS;
