@@ -25,6 +25,7 @@
 #include <string>
 #include "engine.hpp"
 #include "conv_featrows.hpp"
+#include "conv_tile_cost.hpp"
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -485,7 +486,37 @@ static void f16_choose_patch(int Q, int Pn, int kh, int kw, int& tw, int& th)
         }
 }
 
-static bool f16_plan(const cldnn_b200_conv_params& p, F16Plan& pl, std::string* why)
+static bool f16_patch_fits(const cldnn_b200_conv_params& p, int bn, const char** why)
+{
+    auto no = [&](const char* m) { if (why) *why = m; return false; };
+    if (p.stride_x != 1 || p.stride_y != 1 || p.dil_x != 1 || p.dil_y != 1 || p.kh * p.kw == 1) return no("patch mode needs a stride-1 undilated filter larger than 1x1");
+    if (p.ofm > bn) return no("patch mode keeps one feature tile's weights resident: output features within one tile");
+    if ((size_t)p.kh * p.kw * p.in.px * 2 * bn > kF16PatchWeightBytes) return no("patch mode keeps all weights in shared memory: at most 80 KiB");
+    return true;
+}
+
+// The feature tile of an untuned launch by the estimates of conv_tile_cost.hpp; the feature-row form's variant where that is
+// cheaper, else -1.
+static void f16_choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int& bn, int& fr_variant)
+{
+    const int64_t pixels = (int64_t)p.out.b * p.out.y * p.out.x, steps = (int64_t)p.kh * p.kw * (p.in.px * 2 / bk);
+    int64_t m_tiles = (pixels + f16tc::kBM - 1) / f16tc::kBM;
+    if (mode == f16tc::A_TILED) {
+        int bw, bh, bb; f16_choose_box(p.out.x, p.out.y, p.out.b, bw, bh, bb);
+        m_tiles = (int64_t)((p.out.x + bw - 1) / bw) * ((p.out.y + bh - 1) / bh) * ((p.out.b + bb - 1) / bb);
+    }
+    double best = 0.0; bn = 0; fr_variant = -1;
+    for (int b : {64, 128, 256}) {
+        if (b > 64 && b / 2 >= p.ofm) continue;
+        const double t = tile_cost(kTileCostF16, m_tiles, p.ofm, b, steps, bk, TILE_TWO_GROUPS, p.fused_eltw != 0);
+        if (bn == 0 || t < best) { best = t; bn = b; }
+    }
+    int v; const double fr = fr_cost(p, v);
+    if (v >= 0 && fr < best) fr_variant = v;
+}
+
+// `fixed`: the untuned choice that always prepares (what the estimates preferred turned out not to)
+static bool f16_plan(const cldnn_b200_conv_params& p, F16Plan& pl, std::string* why, bool fixed = false)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
     if (p.in.dtype != CLDNN_B200_F16 || p.w_dtype != CLDNN_B200_F16 || p.out.dtype != CLDNN_B200_F16) return no("fp16 activations, weights and output only");
@@ -517,22 +548,28 @@ static bool f16_plan(const cldnn_b200_conv_params& p, F16Plan& pl, std::string* 
                            p.stride_x <= 8 && p.stride_y <= 8 && (int64_t)p.in.b * p.in.pb * 2 >= 131072;
     int mode = -1, bn = 0;
     pl.featrows = false;
-    if (p.tune == 0) {
+    if (p.tune == 0 && !fixed) {
         const int v = fr_inner_product_variant(p);
         if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
     }
     if (p.tune >= kF16TuneFeatRows) { pl.featrows = true; return fr_plan(p, p.tune - kF16TuneFeatRows, pl.fr, why); }
     if (p.tune > 0) { mode = (p.tune - 1) / 3; bn = kF16TuneBN[(p.tune - 1) % 3]; }
-    if (mode < 0) mode = is_1x1_s1 ? f16tc::A_FLAT : (im2col_ok ? f16tc::A_IM2COL : f16tc::A_TILED);
+    if (mode < 0) {
+        mode = is_1x1_s1 ? f16tc::A_FLAT : (im2col_ok ? f16tc::A_IM2COL : f16tc::A_TILED);
+        // resident weights wherever they fit: 64 -> 64 features 3x3 at 224x224, 1 / 32 images, 14.2 against 9.5 us and 264 against 125
+        const int pbn = p.ofm <= 64 ? 64 : (p.ofm <= 128 ? 128 : 256);
+        if (fixed) ;
+        else if (f16_patch_fits(p, pbn, nullptr)) { mode = f16tc::A_PATCH; bn = pbn; }
+        else if (mode != f16tc::A_TILED || tiled_ok) {
+            int v; f16_choose_shape(p, mode, pl.bk, bn, v);
+            if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
+        }
+    }
     if (mode == f16tc::A_FLAT && !is_1x1_s1) return no("flat addressing needs a dense 1x1 stride-1 convolution");
     if (mode == f16tc::A_TILED && !tiled_ok) return no("tiled addressing needs stride 1 or a pointwise filter");
     if (mode == f16tc::A_IM2COL && !im2col_ok) return no("im2col addressing limits exceeded (or tensor below 128 KiB)");
     if (bn == 0) bn = p.ofm > 128 ? 256 : (p.ofm > 64 ? 128 : 64);
-    if (mode == f16tc::A_PATCH) {
-        if (p.stride_x != 1 || p.stride_y != 1 || p.dil_x != 1 || p.dil_y != 1 || p.kh * p.kw == 1) return no("patch mode needs a stride-1 undilated filter larger than 1x1");
-        if (p.ofm > bn) return no("patch mode keeps one feature tile's weights resident: output features within one tile");
-        if ((size_t)p.kh * p.kw * cs * 2 * bn > kF16PatchWeightBytes) return no("patch mode keeps all weights in shared memory: at most 80 KiB");
-    }
+    if (mode == f16tc::A_PATCH) { const char* m = nullptr; if (!f16_patch_fits(p, bn, &m)) return no(m); }
     pl.a_mode = mode; pl.bn = bn; pl.bw = pl.bh = pl.bb = 1;
     if (mode == f16tc::A_TILED) f16_choose_box(p.out.x, p.out.y, p.out.b, pl.bw, pl.bh, pl.bb);
     if (mode == f16tc::A_PATCH) f16_choose_patch(p.out.x, p.out.y, p.kh, p.kw, pl.bw, pl.bh);
@@ -593,11 +630,10 @@ static cudaError_t f16_configure(const Params& P, int max_smem)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
 }
 
-static int32_t f16_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)
+static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out, bool fixed)
 {
-    const cldnn_b200_conv_params& p = *(const cldnn_b200_conv_params*)vp;
     F16Plan pl; std::string why;
-    if (!f16_plan(p, pl, &why)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_f16_tc: " + why);
+    if (!f16_plan(p, pl, &why, fixed)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_f16_tc: " + why);
     if (!a->input0 || !a->output || !a->weights) return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: input, output and weights are required");
     if (p.bias_dtype != CLDNN_B200_NONE && !a->bias) return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: bias_dtype set but no bias pointer");
     if (p.fused_eltw && !p.in_out_opt && !a->input1) return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: fused eltwise needs a second input");
@@ -605,7 +641,10 @@ static int32_t f16_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn
         return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: buffers must be 16-byte aligned");
     if (!f16_driver_entry_points()) return fail(CLDNN_B200_DEVICE_ERROR, "conv_f16_tc: the CUDA driver does not export cuTensorMapEncodeTiled/Im2col");
 
-    if (pl.featrows) return fr_prepare(ctx, p, a, pl.fr, out);
+    if (pl.featrows) {
+        const int32_t st = fr_prepare(ctx, p, a, pl.fr, out);
+        return st != CLDNN_B200_SUCCESS && p.tune == 0 && !fixed ? f16_prepare_as(ctx, p, a, out, true) : st;
+    }
     Params P{};
     P.a_mode = pl.a_mode;
     P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;
@@ -650,7 +689,9 @@ static int32_t f16_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn
     const size_t stage_bytes = (size_t)P.a_stage_bytes + (patch ? 0 : P.b_stage_bytes);
     const size_t staging_total = (size_t)2 * f16tc::kBM * (pl.bn > 128 ? 128 : pl.bn) * 2;   // two unit buffers of up to 128 features
     const size_t aux_bytes = sizeof(f16tc::Aux);
-    if (max_smem < 1024 + aux_bytes + staging_total + resident + 2 * stage_bytes) return fail(CLDNN_B200_OUT_OF_RESOURCES, "conv_f16_tc: not enough shared memory");
+    const bool fits = max_smem >= 1024 + aux_bytes + staging_total + resident + 2 * stage_bytes;
+    if (!fits && p.tune == 0 && !fixed) return f16_prepare_as(ctx, p, a, out, true);
+    if (!fits) return fail(CLDNN_B200_OUT_OF_RESOURCES, "conv_f16_tc: not enough shared memory");
     int stages = (int)((max_smem - 1024 - aux_bytes - staging_total - resident) / stage_bytes);
     if (stages > f16tc::kMaxStages) stages = f16tc::kMaxStages;
     P.stages = stages;
@@ -790,6 +831,11 @@ int32_t f16_batched_gemm_prepare(cldnn_b200_ctx_impl* ctx, const void* A, const 
     B200_CUDA(f16_configure(P, (int)max_smem));
     fn = [P, grid, smem](cudaStream_t s) { return f16_launch(P, grid, smem, s); };
     return CLDNN_B200_SUCCESS;
+}
+
+static int32_t f16_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)
+{
+    return f16_prepare_as(ctx, *(const cldnn_b200_conv_params*)vp, a, out, false);
 }
 
 const KernelDef kdef_conv_f16_tc = {"conv_f16_tc", sizeof(cldnn_b200_conv_params), f16_supports, f16_tune_count, nullptr, f16_prepare};

@@ -13,6 +13,7 @@
 // Launched with programmatic stream serialisation: the weights of the first stages are constants of the network and are
 // requested before the previous kernel has finished; activations only after griddepcontrol.wait.
 #include <cuda.h>
+#include <algorithm>
 #include <mutex>
 #include "conv_featrows.hpp"
 #include "conv_epilogue.cuh"
@@ -389,6 +390,34 @@ int fr_inner_product_variant(const cldnn_b200_conv_params& p)
     return si > 0 ? ci * kFrSplits + si : -1;
 }
 
+// time = launch + (reduction steps of a CTA + epilogue) * (1 + share * CTAs beyond one per SM); constants (us) fitted to every variant of
+// the layers conv_tile_cost.hpp is fitted to (root mean square error 5 %).  More CTAs than are resident at once run in waves, which
+// the other kernels do better: 256 columns leave room for one CTA per SM, and clusters of eight (four) for about 128 (144) of them
+// (fp16 96 -> 256 5x5 at 27x27, 4 images, 256 columns: split of 8, 192 CTAs, 31.0 us; 128 columns, split of 4, 184 CTAs, 18.7).
+double fr_cost(const cldnn_b200_conv_params& p, int& variant)
+{
+    variant = -1;
+    struct Cost { double launch, step, step_row, col, gather, exchange_col, exchange, share; };
+    constexpr Cost kI8 = {4.89, 0.351, 0.00031, 0.0064, 0.0766, 0.0132, 0.893, 0.44}, kF16 = {4.09, 0.338, 0.00039, 0.0061, 0.0844, 0.0072, 1.37, 0.30};
+    const bool f16 = p.in.dtype == CLDNN_B200_F16;
+    const Cost& c = f16 ? kF16 : kI8;
+    const int64_t cs = p.in.px * (f16 ? 2 : 1), pixels = (int64_t)p.out.b * p.out.y * p.out.x;
+    const int64_t bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32), steps = (int64_t)p.kh * p.kw * (cs / bk), m_tiles = (p.ofm + kRows - 1) / kRows;
+    double best = 0.0;
+    for (int v = 0; v < kFrVariants; ++v) {
+        FrPlan pl;
+        const int64_t cols = kCols[v / kFrSplits], split = 1 << (v % kFrSplits), ctas = m_tiles * ((pixels + cols - 1) / cols) * split;
+        const int64_t resident = (split == 8 ? 128 : (split == 4 ? 144 : 148)) * (cols == 256 ? 1 : 2);
+        if (ctas > resident || !fr_plan(p, v, pl, nullptr)) continue;
+        const double valid = (double)std::min(cols, pixels);
+        const double main = (double)((steps + split - 1) / split) * (c.step + c.step_row * (double)(kRows + cols) * ((double)bk / 128.0));
+        const double epi = c.col * (double)cols + c.gather * valid / (double)split + (split > 1 ? c.exchange_col * valid + c.exchange : 0.0);
+        const double t = c.launch + (main + epi) * (1.0 + c.share * std::max(0.0, (double)ctas / 148.0 - 1.0));
+        if (variant < 0 || t < best) { best = t; variant = v; }
+    }
+    return best;
+}
+
 int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, const cldnn_b200_args* a, const FrPlan& pl, cldnn_b200_prepared_impl* out)
 {
     if (!fr_entry_points()) return fail(CLDNN_B200_DEVICE_ERROR, "conv_featrows: the CUDA driver does not export cuTensorMapEncodeTiled/Im2col");
@@ -432,10 +461,13 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     P.quant = a->weights_quantization_factors; P.calib = a->output_calibration_factors; P.ecal = a->eltw_output_calibration_factors;
     P.status = ctx->d_status; P.epi = make_epi_cfg(p);
 
-    // Operand ring: every step of a CTA in flight at once where that fits.  More CTAs than SMs: two share an SM.
+    // Operand ring: every step of a CTA in flight at once where that fits.  More CTAs than SMs: two share an SM.  Clusters of four or
+    // eight do not fill a GPC evenly, so with one CTA per SM a part of them would wait for a second wave well before the SMs run
+    // out (8-bit 512 -> 512 3x3 at 4 images, 16 clusters of eight, ring of five 24 KiB stages: 17.2 us against 10.1 in twice as many CTAs).
     const size_t dump = (size_t)P.cols * kRows * 4, stage = (size_t)P.a_stage_bytes + P.b_stage_bytes;
     const size_t max_smem = (size_t)ctx->prop.sharedMemPerBlockOptin, other = 1024 + sizeof(FrAux);
-    size_t budget = ctas > ctx->prop.multiProcessorCount ? (ctx->prop.sharedMemPerMultiprocessor / 2) - 2048 : max_smem;
+    const int64_t alone = P.split >= 4 ? ctx->prop.multiProcessorCount / 2 : ctx->prop.multiProcessorCount;
+    size_t budget = ctas > alone ? (ctx->prop.sharedMemPerMultiprocessor / 2) - 2048 : max_smem;
     if (budget < other + dump || budget < other + 2 * stage) budget = max_smem;
     if (budget < other + dump || budget < other + 2 * stage) return fail(CLDNN_B200_OUT_OF_RESOURCES, "conv_featrows: not enough shared memory");
     const int most = (P.k_steps + P.split - 1) / P.split;

@@ -20,6 +20,9 @@ constexpr int kFrVariants = kFrCols * kFrSplits;
 bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::string* why);
 // The variant an untuned inner product (a pointwise convolution of 1x1 maps) takes; -1: the pixel-row kernels are the better choice.
 int fr_inner_product_variant(const cldnn_b200_conv_params& p);
+// The variant with the lowest expected time (us, returned) for a convolution of any shape, among those whose CTAs are
+// all resident at once; -1: none.
+double fr_cost(const cldnn_b200_conv_params& p, int& variant);
 int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, const cldnn_b200_args* a, const FrPlan& pl, cldnn_b200_prepared_impl* out);
 
 }  // namespace b200

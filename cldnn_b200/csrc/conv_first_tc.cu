@@ -481,6 +481,11 @@ static bool ftc_plan(const cldnn_b200_conv_params& p, std::string* why)
 // tuning variants: 0 / 1 the gather kernel of this file; 2 / 3 the row form of conv_i8_first_rows.cu (fp16 here; 8-bit layers reach
 // it through conv_i8_first) with two / four epilogue warp groups
 static bool ftc_rows(const cldnn_b200_conv_params& p) { return p.tune >= 2 && p.in.dtype == CLDNN_B200_F16; }
+// Untuned fp16: the row form from an image of 128x128 on (3x3 -> 64 at 224x224, gather / row form: 17.5 / 8.4 us at 1 image, 153 / 61 at 32)
+static bool ftc_prefers_rows(const cldnn_b200_conv_params& p)
+{
+    return p.tune == 0 && p.in.dtype == CLDNN_B200_F16 && (int64_t)p.out.b * p.out.y * p.out.x >= 16384 && first_rows_plan(p, nullptr);
+}
 static bool ftc_supports(const void* vp)
 {
     const cldnn_b200_conv_params& p = *(const cldnn_b200_conv_params*)vp;
@@ -494,7 +499,8 @@ static size_t ftc_scratch(const void* vp)
 {
     const auto& p = *(const cldnn_b200_conv_params*)vp;
     if (ftc_rows(p)) return first_rows_scratch(p);
-    return ftc_table_offset(p) + (size_t)ftc_cores(p) * 2 * sizeof(int4);
+    const size_t gather = ftc_table_offset(p) + (size_t)ftc_cores(p) * 2 * sizeof(int4);
+    return ftc_prefers_rows(p) ? std::max(gather, first_rows_scratch(p)) : gather;
 }
 
 static int32_t ftc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)
@@ -504,6 +510,8 @@ static int32_t ftc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn
         if (!ftc_rows(pr)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_first_tc: the row form is the fp16 variant here");
         return first_rows_prepare(ctx, pr, a, out, pr.tune == 3 ? 4 : 2);
     }
+    if (ftc_prefers_rows(*(const cldnn_b200_conv_params*)vp) && first_rows_fits(*(const cldnn_b200_conv_params*)vp, a))
+        return first_rows_prepare(ctx, *(const cldnn_b200_conv_params*)vp, a, out, 2);
     const cldnn_b200_conv_params p = simplified_conv_params(*(const cldnn_b200_conv_params*)vp);
     std::string why;
     if (!ftc_plan(p, &why)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_first_tc: " + why);
@@ -511,7 +519,7 @@ static int32_t ftc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn
     if (p.bias_dtype != CLDNN_B200_NONE && !a->bias) return fail(CLDNN_B200_INVALID_ARG, "conv_first_tc: bias_dtype set but no bias pointer");
     if (p.quantization && !a->weights_quantization_factors) return fail(CLDNN_B200_INVALID_ARG, "conv_first_tc: quantization set but no factors");
     if (p.calibration && !a->output_calibration_factors) return fail(CLDNN_B200_INVALID_ARG, "conv_first_tc: calibration set but no factors");
-    const size_t need = ftc_scratch(&p);
+    const size_t need = ftc_table_offset(p) + (size_t)ftc_cores(p) * 2 * sizeof(int4);
     if (!a->scratch || a->scratch_bytes < need) return fail(CLDNN_B200_INVALID_ARG, "conv_first_tc: needs " + std::to_string(need) + " bytes of scratch for the packed weights");
     if (((uintptr_t)a->scratch | (uintptr_t)a->output) & 15) return fail(CLDNN_B200_INVALID_ARG, "conv_first_tc: scratch and output must be 16-byte aligned");
     const bool half = p.in.dtype == CLDNN_B200_F16;

@@ -400,12 +400,20 @@ static bool first_supports(const void* vp)
 // 4, 5: the row form (conv_i8_first_rows.cu: output rows as GEMM rows, the raw image rows as the TMA-loaded operand) with two / four
 // epilogue warp groups
 static int first_tune_count(const void*) { return 6; }
+// Untuned: the row form where there are enough pixels to amortise each CTA's copy of its banded matrices (up to 168 KB).  7x7/2 -> 64 at
+// 224x224, general / row form: 10.6 / 11.0 us at 4 images (50 k pixels), 14.6 / 13.1 at 8, 239 / 111 at 256; 7x7/2 at 160x160, 8 / 13
+// images (51 / 83 k): 10.8 / 12.0 and 13.6 / 12.8; 3x3/2 -> 32 at 192x192, 4 / 8 images (37 / 74 k): 7.5 / 7.7 and 9.2 / 8.2.
+static bool first_prefers_rows(const cldnn_b200_conv_params& p)
+{
+    return p.tune == 0 && (int64_t)p.out.b * p.out.y * p.out.x >= 65536 && first_rows_plan(simplified_conv_params(p), nullptr);
+}
 static int first_kp(const cldnn_b200_conv_params& p) { return (p.ifm * p.kh * 8 + 31) / 32 * 32; }
 static size_t first_scratch(const void* vp)
 {
     const auto& p = *(const cldnn_b200_conv_params*)vp;
+    const size_t general = (size_t)p.ofm * first_kp(p);
     if (p.tune >= kTuneRows) return first_rows_scratch(p);
-    return (size_t)p.ofm * first_kp(p);
+    return first_prefers_rows(p) ? std::max(general, first_rows_scratch(p)) : general;
 }
 
 // Validates the arguments and fills the launch constants; `wpacked` is where the packed weights will live.
@@ -419,7 +427,7 @@ static int32_t first_setup(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_param
     if (p.bias_dtype != CLDNN_B200_NONE && !a->bias) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_first: bias_dtype set but no bias pointer");
     if (p.quantization && !a->weights_quantization_factors) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_first: quantization set but no factors");
     if (p.calibration && !a->output_calibration_factors) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_first: calibration set but no factors");
-    const size_t need = first_scratch(&p);
+    const size_t need = (size_t)p.ofm * first_kp(p);
     if (!wpacked || wpacked_bytes < need) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_first: needs " + std::to_string(need) + " bytes of scratch for the packed weights");
     if (((uintptr_t)wpacked | (uintptr_t)a->output) & 15) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_first: scratch and output must be 16-byte aligned");
 
@@ -486,6 +494,7 @@ static int32_t first_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cld
 {
     const cldnn_b200_conv_params& p = *(const cldnn_b200_conv_params*)vp;
     if (p.tune >= kTuneRows) return first_rows_prepare(ctx, p, a, out, p.tune == kTuneRows + 1 ? 4 : 2);
+    if (first_prefers_rows(p) && first_rows_fits(p, a)) return first_rows_prepare(ctx, p, a, out, 4);
     FirstParams P; int grid = 0; size_t smem = 0;
     const int32_t st = first_setup(ctx, p, a, a->scratch, a->scratch_bytes, P, grid, smem);
     if (st != CLDNN_B200_SUCCESS) return st;

@@ -68,6 +68,10 @@ struct RowsParams {
     uint8_t* out; const void* bias; const float* quant;
     uint32_t* status;
     EpiCfg epi;
+    // fp16 path: the image and the banded matrices again, for pixels whose sums have to be taken tap by tap
+    const __half* in; const __half* banded;
+    int64_t in_pb, in_pf, in_py;
+    int32_t H, W, kw, stride, pad_x, pad_y, off[2];
 };
 
 struct RowsAux {
@@ -184,19 +188,51 @@ __device__ __forceinline__ float rows_act(int32_t fn, float x, float m, float n)
     return rows_act_other(fn, x, m, n);
 }
 
+// 32 features of one output pixel tap by tap.  A window of the row form reaches past the taps of a pixel, and the zeros of the
+// banded matrices there turn an Inf or NaN of the image into NaN; the same goes for zero-filled pixels outside the image under
+// weights that are not finite.  A sum that came out NaN is therefore taken again over the pixel's own taps inside the image.
+__device__ __noinline__ void rows_pixel_f16(const RowsParams& P, const RowsAux* aux, int v, int n, int y, int x, int i, int f0, uint8_t* dst)
+{
+    const __half* img = P.in + (int64_t)n * P.in_pb;
+    const int KW = 16, tap0 = P.off[v] + P.stride * i;
+    for (int j = 0; j < 32; ++j) {
+        float acc = 0.0f;
+        for (int ky = 0; ky < P.kh; ++ky) {
+            const int iy = y * P.stride - P.pad_y + ky;
+            if (iy < 0 || iy >= P.H) continue;
+            for (int c = 0; c < P.C; ++c) {
+                const __half* w = P.banded + ((int64_t)(v * P.kh * P.C + ky * P.C + c) * kRCols + i * P.ofm + f0 + j) * KW + tap0;
+                const __half* row = img + c * P.in_pf + iy * P.in_py;
+                for (int kx = 0; kx < P.kw; ++kx) {
+                    const int ix = x * P.stride - P.pad_x + kx;
+                    if (ix >= 0 && ix < P.W) acc = fmaf(__half2float(row[ix]), __half2float(w[kx]), acc);
+                }
+            }
+        }
+        reinterpret_cast<__half*>(dst)[j] = __float2half_rn(rows_act(P.act, acc + aux->bias_f[f0 + j], P.act_m, P.act_n));
+    }
+}
+
 // fp16: fp32 accumulators + bias -> activation -> one rounding to half; 32 columns = 64 output bytes per trip
 __device__ __forceinline__ void rows_epi_f16(const RowsParams& P, const RowsAux* aux, uint32_t t_row, uint8_t* out_row, bool row_ok, int x_left,
-                                             uint32_t tmem_empty_bar, int lane, int c_lo, int c_hi)
+                                             uint32_t tmem_empty_bar, int lane, int c_lo, int c_hi, int v, int n, int y, int x0)
 {
     const bool st32 = P.st32 != 0;
 #pragma unroll 1
     for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
         uint32_t r[32];
+        __syncwarp();
         tmem_ld_32x32(t_row + (uint32_t)c0, r);
         tmem_ld_wait();
         if (c0 + 32 >= c_hi) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(tmem_empty_bar); }
         const int i = c0 >> P.ofm_shift, f0 = c0 & (P.ofm - 1);
         if (row_ok && i < x_left) {
+            // any NaN among the 32 sums makes their sum NaN (so does Inf - Inf, which only costs the slower path)
+            float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < 32; ++j) s[j & 3] += __uint_as_float(r[j]);
+            const float total = (s[0] + s[1]) + (s[2] + s[3]);
+            if (total != total) { rows_pixel_f16(P, aux, v, n, y, x0 + i, i, f0, out_row + (int64_t)i * P.out_px + 2 * f0); continue; }
             uint4 o[4];
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
@@ -366,7 +402,7 @@ conv_i8_first_rows_kernel(const __grid_constant__ RowsParams P)
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kRCols);
             const uint32_t te = smem_u32(&aux->tmem_empty[acc]);
-            if (kHalf) rows_epi_f16(P, aux, t_row, out_row, row_ok, x_left, te, lane, c_lo, c_hi);
+            if (kHalf) rows_epi_f16(P, aux, t_row, out_row, row_ok, x_left, te, lane, c_lo, c_hi, v, t.n, y, x0);
             else if (wide) rows_epi_tile_wide(P, aux, t_row, out_row, row_ok, x_left, te, lane, c_lo, c_hi);
             else if (G == 4) switch (P.mode) {
                 case 0: rows_epi_half<0, false>(P, aux, t_row, out_row, row_ok, x_left, te, lane, c_lo); break;
@@ -479,6 +515,12 @@ bool first_rows_plan(const cldnn_b200_conv_params& p, std::string* why)
 
 size_t first_rows_scratch(const cldnn_b200_conv_params& p) { return (size_t)2 * p.ifm * p.kh * kRCols * 32; }
 
+bool first_rows_fits(const cldnn_b200_conv_params& p, const cldnn_b200_args* a)
+{
+    return a->input0 && a->output && a->weights && a->scratch && a->scratch_bytes >= first_rows_scratch(p) &&
+           !(((uintptr_t)a->scratch | (uintptr_t)a->output | (uintptr_t)a->input0) & 15);
+}
+
 int32_t first_rows_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p_in, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out, int groups)
 {
     const bool half = p_in.in.dtype == CLDNN_B200_F16;
@@ -527,6 +569,11 @@ int32_t first_rows_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_param
     P.out = (uint8_t*)a->output; P.bias = a->bias; P.quant = a->weights_quantization_factors;
     P.status = ctx->d_status;
     P.groups = groups == 4 ? 4 : 2;
+    if (half) {
+        P.in = (const __half*)a->input0 + p.in.offset; P.banded = (const __half*)a->scratch;
+        P.in_pb = p.in.pb; P.in_pf = p.in.pf; P.in_py = p.in.py; P.H = p.in.y; P.W = p.in.x;
+        P.kw = p.kw; P.stride = p.stride_x; P.pad_x = p.pad_x; P.pad_y = p.pad_y; P.off[0] = g.off[0]; P.off[1] = g.off[1];
+    }
 
     const CUtensorMapDataType dt = half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
     for (int r = 0; r < g.planes; ++r) {

@@ -26,6 +26,7 @@
 #include <mutex>
 #include "conv_i8_tc.hpp"
 #include "conv_featrows.hpp"
+#include "conv_tile_cost.hpp"
 #include "conv_epilogue.cuh"
 
 namespace b200 {
@@ -461,7 +462,42 @@ static void choose_patch(int Q, int Pn, int kh, int kw, int& tw, int& th)
     }
 }
 
-static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* why)
+// The tile shape of an untuned launch in the common configuration (the specialised kernel's), by the estimates of
+// conv_tile_cost.hpp; -1 in `fr_variant` unless the feature-row form is the cheapest.
+static void choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int& bn, int& groups, int& pair, int& fr_variant)
+{
+    const int64_t cs = p.in.px, pixels = (int64_t)p.out.b * p.out.y * p.out.x;
+    int64_t m_tiles = (pixels + kBM - 1) / kBM;
+    if (mode == A_TILED) {
+        int bw, bh, bb; choose_box(p.out.x, p.out.y, p.out.b, bw, bh, bb);
+        m_tiles = (int64_t)((p.out.x + bw - 1) / bw) * ((p.out.y + bh - 1) / bh) * ((p.out.b + bb - 1) / bb);
+    }
+    fr_variant = -1; groups = 2; pair = 0;
+    if (p.ofm <= 32) {
+        // a 32-feature tile (the general kernel) is quicker through a single tile, the specialised kernel through many:
+        // 32 -> 16 features at 112x112, 8 / 128 images: 9.7 against 7.8 us, 88 against 58
+        bn = m_tiles > 2 * kCostSMs ? 64 : 32; groups = bn == 64 ? 4 : 2;
+        return;
+    }
+    double best = 0.0; bn = 0;
+    for (int b : {64, 128, 256}) {
+        if (b > 64 && b / 2 >= p.ofm) continue;
+        const bool half_steps = b == 256 && p.fused_eltw && bk == 128 && cs < 512;     // as tc_plan sets the stage size
+        const int kb = half_steps ? 64 : bk;
+        const int64_t steps = (int64_t)p.kh * p.kw * (cs / kb);
+        for (TileKind k : {TILE_TWO_GROUPS, TILE_FOUR_GROUPS, TILE_PAIR}) {
+            if (k == TILE_FOUR_GROUPS && b == 256) continue;
+            if (k == TILE_PAIR && (b == 64 || p.ofm % b || pixels < 2 * kBM)) continue;
+            const double t = tile_cost(kTileCostI8, m_tiles, p.ofm, b, steps, kb, k, p.fused_eltw != 0);
+            if (bn == 0 || t < best) { best = t; bn = b; groups = k == TILE_FOUR_GROUPS ? 4 : 2; pair = k == TILE_PAIR; }
+        }
+    }
+    int v; const double fr = fr_cost(p, v);
+    if (v >= 0 && fr < best) fr_variant = v;
+}
+
+// `fixed`: the untuned choice is the one that suits every epilogue (the specialised kernel turned out not to take the launch)
+static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* why, bool fixed = false)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
     if (!is_int8(p.in.dtype)) return no("activations must be u8 or i8");
@@ -499,7 +535,7 @@ static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* wh
     int tune = p.tune;
     int mode = -1, bn = 0;
     pl.epi_groups = 2; pl.pair = 0; pl.featrows = false;
-    if (tune == 0) {
+    if (tune == 0 && !fixed) {
         const int v = fr_inner_product_variant(p);
         if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
     }
@@ -539,7 +575,15 @@ static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* wh
     if (mode < 0) {
         const int fbn = p.ofm % 256 == 0 ? 256 : (p.ofm % 128 == 0 ? 128 : 64);
         if (!patch_why(fbn)) { mode = A_PATCH; bn = fbn; }
-        else mode = is_1x1_s1 ? A_FLAT : (im2col_ok ? A_IM2COL : A_TILED);
+        else {
+            mode = is_1x1_s1 ? A_FLAT : (im2col_ok ? A_IM2COL : A_TILED);
+            auto aligned = [](const cldnn_b200_tensor& t) { return t.pf == 1 && t.px % 16 == 0 && t.py % 16 == 0 && t.pb % 16 == 0 && t.offset % 16 == 0; };
+            if (p.tune == 0 && !fixed && lean_params(p) && aligned(p.out) && (!p.fused_eltw || aligned(p.in_out_opt ? p.out : p.eltw)) && (mode != A_TILED || tiled_ok)) {
+                int v;
+                choose_shape(p, mode, pl.bk, bn, pl.epi_groups, pl.pair, v);
+                if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
+            }
+        }
     }
     if (mode == A_FLAT && !is_1x1_s1) return no("flat addressing needs a dense 1x1 stride-1 convolution");
     if (mode == A_TILED && !tiled_ok) return no("tiled addressing needs stride 1 or a pointwise filter");
@@ -583,11 +627,10 @@ static CUresult encode_pixel_map(CUtensorMap* tm, const TcPlan& pl, void* ptr, c
                           CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-static int32_t tc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)
+static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out, bool fixed)
 {
-    const cldnn_b200_conv_params p = simplified_conv_params(*(const cldnn_b200_conv_params*)vp);
     TcPlan pl; std::string why;
-    if (!tc_plan(p, pl, &why)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: " + why);
+    if (!tc_plan(p, pl, &why, fixed)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: " + why);
     if (!a->input0 || !a->output || !a->weights) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: input, output and weights are required");
     if (p.bias_dtype != CLDNN_B200_NONE && !a->bias) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: bias_dtype set but no bias pointer");
     if (p.quantization && !a->weights_quantization_factors) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: quantization set but no factors");
@@ -597,7 +640,10 @@ static int32_t tc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_
     if (((uintptr_t)a->input0 | (uintptr_t)a->weights) & 15) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: input and weights must be 16-byte aligned");
     if (!load_driver_entry_points()) return fail(CLDNN_B200_DEVICE_ERROR, "conv_i8_tc: the CUDA driver does not export cuTensorMapEncodeTiled/Im2col");
 
-    if (pl.featrows) return fr_prepare(ctx, p, a, pl.fr, out);
+    if (pl.featrows) {
+        const int32_t st = fr_prepare(ctx, p, a, pl.fr, out);
+        return st != CLDNN_B200_SUCCESS && p.tune == 0 && !fixed ? tc_prepare_as(ctx, p, a, out, true) : st;
+    }
     TcParams P{};
     P.a_mode = pl.a_mode;
     P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;
@@ -679,6 +725,7 @@ static int32_t tc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_
     P.acc_bound = (float)p.kh * (float)p.kw * (float)p.ifm * (p.in.dtype == CLDNN_B200_U8 ? 255.0f : 128.0f) * 128.0f;
     P.epi_groups = pl.epi_groups;
     const bool use_fast = (p.tune <= 12 || p.tune > 24) && tc_fast_eligible(P);
+    if (!use_fast && p.tune == 0 && !fixed && pl.a_mode != A_PATCH) return tc_prepare_as(ctx, p, a, out, true);
     if (pl.pair && !use_fast) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: CTA pairs exist on the specialised kernel only");
     if (pl.epi_groups > 2 && !use_fast) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: four epilogue groups exist on the specialised kernel only");
 
@@ -806,6 +853,11 @@ static int32_t tc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_
         out->fn = [P, grid, smem](cudaStream_t s) { conv_i8_tc_kernel<<<grid, kThreads, smem, s>>>(P); return cudaGetLastError(); };
     out->launches = 1;
     return CLDNN_B200_SUCCESS;
+}
+
+static int32_t tc_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)
+{
+    return tc_prepare_as(ctx, simplified_conv_params(*(const cldnn_b200_conv_params*)vp), a, out, false);
 }
 
 const KernelDef kdef_conv_i8_tc = {"conv_i8_tc", sizeof(cldnn_b200_conv_params), tc_supports, tc_tune_count, nullptr, tc_prepare};
