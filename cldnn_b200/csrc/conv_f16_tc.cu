@@ -63,6 +63,7 @@ struct alignas(64) Params {
     int32_t b_total_bytes, patch_alloc;      // patch mode: all taps' weights (resident), bytes reserved per patch
     int32_t batch_tiles;                     // batched GEMM view: tiles per batch, the weight 'tap' is the batch index (0 = plain convolution)
     int32_t ofm, fused, bias_dtype, act, eltw_act;
+    int32_t group_tiles, group_ch;           // grouped: feature tiles per group (0: one group), its input features
     float act_m, act_n, eltw_m, eltw_n;
     const void* bias;
     uint32_t* status;
@@ -218,21 +219,22 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
                     const int tw = m_tile % P.tiles_w; const int t2 = m_tile / P.tiles_w;
                     c_w = tw * P.bw - P.pad_x; c_h = (t2 % P.tiles_h) * P.bh - P.pad_y; c_n = (t2 / P.tiles_h) * P.bb;
                 }
+                const int g0 = P.group_tiles ? n_tile / P.group_tiles * P.group_ch : 0;      // first input feature of the tile's group
                 int tap = P.batch_tiles ? m_tile / P.batch_tiles : 0, cc = 0, r = 0, s = 0;
                 for (int ks = 0; ks < P.k_steps; ++ks) {
                     if (!__all_sync(0xffffffffu, mbar_wait_lean(smem_u32(&aux->empty[stage]), phase ^ 1u, s_abort, P.status, kErr))) { ok = false; break; }
                     const uint32_t full = smem_u32(&aux->full[stage]);
                     const uint32_t a_dst = a_base + (uint32_t)(stage * P.a_stage_bytes);
                     const uint32_t b_dst = b_base + (uint32_t)(stage * P.b_stage_bytes);
-                    const int c0 = cc * bke;
+                    const int c0 = cc * bke, a0 = g0 + c0;
                     if (leader && patch) {
                         mbar_expect_tx(full, (uint32_t)P.a_tx_bytes);
                         for (int sc = 0; sc < P.kw; ++sc) tma_load_4d(a_dst + (uint32_t)(sc * P.patch_alloc), &P.tmA, full, c0, c_w + sc, c_h, c_n);
                     } else if (leader) {
                         mbar_expect_tx(full, (uint32_t)(P.a_tx_bytes + P.b_tx_bytes));
-                        if (P.a_mode == A_FLAT) tma_load_2d(a_dst, &P.tmA, full, c0, m_tile * kBM);
-                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d(a_dst, &P.tmA, full, c0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
-                        else tma_load_4d(a_dst, &P.tmA, full, c0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
+                        if (P.a_mode == A_FLAT) tma_load_2d(a_dst, &P.tmA, full, a0, m_tile * kBM);
+                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d(a_dst, &P.tmA, full, a0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
+                        else tma_load_4d(a_dst, &P.tmA, full, a0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
                         tma_load_3d(b_dst, &P.tmB, full, c0, tap, n_tile * BN);
                     }
                     ++issued;
@@ -489,6 +491,7 @@ static void f16_choose_patch(int Q, int Pn, int kh, int kw, int& tw, int& th)
 static bool f16_patch_fits(const cldnn_b200_conv_params& p, int bn, const char** why)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
+    if (p.groups > 1) return no("patch mode reads all input features");
     if (p.stride_x != 1 || p.stride_y != 1 || p.dil_x != 1 || p.dil_y != 1 || p.kh * p.kw == 1) return no("patch mode needs a stride-1 undilated filter larger than 1x1");
     if (p.ofm > bn) return no("patch mode keeps one feature tile's weights resident: output features within one tile");
     if ((size_t)p.kh * p.kw * p.in.px * 2 * bn > kF16PatchWeightBytes) return no("patch mode keeps all weights in shared memory: at most 80 KiB");
@@ -499,7 +502,7 @@ static bool f16_patch_fits(const cldnn_b200_conv_params& p, int bn, const char**
 // cheaper, else -1.
 static void f16_choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int& bn, int& fr_variant)
 {
-    const int64_t pixels = (int64_t)p.out.b * p.out.y * p.out.x, steps = (int64_t)p.kh * p.kw * (p.in.px * 2 / bk);
+    const int64_t pixels = (int64_t)p.out.b * p.out.y * p.out.x, steps = (int64_t)p.kh * p.kw * (reduction_features(p) * 2 / bk);
     int64_t m_tiles = (pixels + f16tc::kBM - 1) / f16tc::kBM;
     if (mode == f16tc::A_TILED) {
         int bw, bh, bb; f16_choose_box(p.out.x, p.out.y, p.out.b, bw, bh, bb);
@@ -507,7 +510,7 @@ static void f16_choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, 
     }
     double best = 0.0; bn = 0; fr_variant = -1;
     for (int b : {64, 128, 256}) {
-        if (b > 64 && b / 2 >= p.ofm) continue;
+        if (p.groups > 1 ? b != 128 : (b > 64 && b / 2 >= p.ofm)) continue;      // (a grouped tile lies inside its group)
         const double t = tile_cost(kTileCostF16, m_tiles, p.ofm, b, steps, bk, TILE_TWO_GROUPS, p.fused_eltw != 0);
         if (bn == 0 || t < best) { best = t; bn = b; }
     }
@@ -516,19 +519,20 @@ static void f16_choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, 
 }
 
 // `fixed`: the untuned choice that always prepares (what the estimates preferred turned out not to)
-static bool f16_plan(const cldnn_b200_conv_params& p, F16Plan& pl, std::string* why, bool fixed = false)
+static bool f16_plan(const cldnn_b200_conv_params& p_in, F16Plan& pl, std::string* why, bool fixed = false)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
+    cldnn_b200_conv_params p = p_in;
+    if (!grouped_view(p, why)) return false;
     if (p.in.dtype != CLDNN_B200_F16 || p.w_dtype != CLDNN_B200_F16 || p.out.dtype != CLDNN_B200_F16) return no("fp16 activations, weights and output only");
-    if (p.groups != 1) return no("grouped convolution is handled by other kernels");
     if (p.quantization || p.calibration || p.has_o_qf) return no("no quantisation on the fp16 path");
     if (p.kh < 1 || p.kw < 1 || p.kh * p.kw > 255 || p.stride_x < 1 || p.stride_y < 1 || p.dil_x < 1 || p.dil_y < 1) return no("filter geometry");
-    if (p.out.f != p.ofm || p.in.f != p.ifm) return no("feature counts");
+    if (p.out.f != p.ofm || p.in.f != p.ifm * p.groups) return no("feature counts");
     // pitches are in elements
     if (p.in.pf != 1 || p.in.px % 16 || p.in.py % 8 || p.in.pb % 8 || p.in.offset % 8 || p.in.px < p.in.f || p.in.py < p.in.px * p.in.x || p.in.pb < p.in.py * p.in.y)
         return no("input must be byxf with the stored feature count a multiple of 16");
     if (p.out.pf != 1 || p.out.px % 8 || p.out.py % 8 || p.out.pb % 8 || p.out.offset % 8) return no("output must be byxf with 16-byte aligned pitches");
-    if (p.w_pi != 1 || p.w_px != p.in.px || p.w_py != p.w_px * p.kw || p.w_po % 8 || p.w_offset % 8) return no("weights must be oyxi with the input's stored feature count");
+    if (p.w_pi != 1 || (p.groups == 1 && p.w_px != p.in.px) || p.w_py != p.w_px * p.kw || p.w_po % 8 || p.w_offset % 8) return no("weights must be oyxi with the input's stored feature count");
     if (p.bias_dtype != CLDNN_B200_NONE && p.bias_dtype != CLDNN_B200_F16 && p.bias_dtype != CLDNN_B200_F32) return no("bias type");
     if (p.fused_eltw) {
         const cldnn_b200_tensor& e = p.in_out_opt ? p.out : p.eltw;
@@ -539,7 +543,7 @@ static bool f16_plan(const cldnn_b200_conv_params& p, F16Plan& pl, std::string* 
     const int Q_ = (p.in.x + 2 * p.pad_x - ((p.kw - 1) * p.dil_x + 1)) / p.stride_x + 1;
     if (p.out.y != P_ || p.out.x != Q_ || p.out.b != p.in.b) return no("output size does not match the sliding-window rule");
 
-    const int cs = (int)p.in.px;                                    // stored channels
+    const int cs = (int)reduction_features(p);                      // stored channels
     pl.bk = cs % 64 == 0 ? 128 : (cs % 32 == 0 ? 64 : 32);          // bytes of K per stage
     const bool is_1x1_s1 = p.kh == 1 && p.kw == 1 && p.stride_x == 1 && p.stride_y == 1 && p.pad_x == 0 && p.pad_y == 0 && f16_dense(p.in);
     const bool pointwise = p.kh == 1 && p.kw == 1 && p.pad_x == 0 && p.pad_y == 0;
@@ -568,6 +572,8 @@ static bool f16_plan(const cldnn_b200_conv_params& p, F16Plan& pl, std::string* 
     if (mode == f16tc::A_FLAT && !is_1x1_s1) return no("flat addressing needs a dense 1x1 stride-1 convolution");
     if (mode == f16tc::A_TILED && !tiled_ok) return no("tiled addressing needs stride 1 or a pointwise filter");
     if (mode == f16tc::A_IM2COL && !im2col_ok) return no("im2col addressing limits exceeded (or tensor below 128 KiB)");
+    if (p.groups > 1 && bn == 0) bn = 128;
+    if (p.groups > 1 && p.ofm / p.groups % bn) return no("grouped convolution: a feature tile must lie inside one group");
     if (bn == 0) bn = p.ofm > 128 ? 256 : (p.ofm > 64 ? 128 : 64);
     if (mode == f16tc::A_PATCH) { const char* m = nullptr; if (!f16_patch_fits(p, bn, &m)) return no(m); }
     pl.a_mode = mode; pl.bn = bn; pl.bw = pl.bh = pl.bb = 1;
@@ -630,10 +636,12 @@ static cudaError_t f16_configure(const Params& P, int max_smem)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
 }
 
-static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out, bool fixed)
+static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p_in, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out, bool fixed)
 {
     F16Plan pl; std::string why;
-    if (!f16_plan(p, pl, &why, fixed)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_f16_tc: " + why);
+    if (!f16_plan(p_in, pl, &why, fixed)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_f16_tc: " + why);
+    cldnn_b200_conv_params p = p_in;
+    grouped_view(p, nullptr);
     if (!a->input0 || !a->output || !a->weights) return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: input, output and weights are required");
     if (p.bias_dtype != CLDNN_B200_NONE && !a->bias) return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: bias_dtype set but no bias pointer");
     if (p.fused_eltw && !p.in_out_opt && !a->input1) return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: fused eltwise needs a second input");
@@ -643,13 +651,14 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
 
     if (pl.featrows) {
         const int32_t st = fr_prepare(ctx, p, a, pl.fr, out);
-        return st != CLDNN_B200_SUCCESS && p.tune == 0 && !fixed ? f16_prepare_as(ctx, p, a, out, true) : st;
+        return st != CLDNN_B200_SUCCESS && p.tune == 0 && !fixed ? f16_prepare_as(ctx, p_in, a, out, true) : st;
     }
     Params P{};
     P.a_mode = pl.a_mode;
     P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;
     P.kh = p.kh; P.kw = p.kw; P.stride_x = p.stride_x; P.stride_y = p.stride_y; P.pad_x = p.pad_x; P.pad_y = p.pad_y; P.dil_x = p.dil_x; P.dil_y = p.dil_y;
-    const int cs = (int)p.in.px;
+    const int cs = (int)reduction_features(p);
+    const cuuint64_t a_features = (cuuint64_t)p.in.px;               // of the activations' tensor map
     const int bke = pl.bk / 2;
     P.bk = pl.bk; P.chunks = cs / bke; P.k_steps = p.kh * p.kw * P.chunks;
     P.bn = pl.bn; P.n_tiles = (p.ofm + pl.bn - 1) / pl.bn;
@@ -680,6 +689,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     P.idesc = (1u << 4) | ((uint32_t)(pl.bn >> 3) << 17) | ((uint32_t)(f16tc::kBM >> 4) << 24);
     const int nbuf = pl.bn >= 256 ? 2 : 4;
     P.tmem_cols = (uint32_t)(nbuf * pl.bn);
+    if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / pl.bn; P.group_ch = p.ifm; }
     P.ofm = p.ofm; P.fused = p.fused_eltw; P.bias_dtype = p.bias_dtype; P.act = p.act; P.eltw_act = p.eltw_act;
     P.act_m = p.act_m; P.act_n = p.act_n; P.eltw_m = p.eltw_m; P.eltw_n = p.eltw_n;
     P.bias = a->bias; P.status = ctx->d_status;
@@ -690,7 +700,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     const size_t staging_total = (size_t)2 * f16tc::kBM * (pl.bn > 128 ? 128 : pl.bn) * 2;   // two unit buffers of up to 128 features
     const size_t aux_bytes = sizeof(f16tc::Aux);
     const bool fits = max_smem >= 1024 + aux_bytes + staging_total + resident + 2 * stage_bytes;
-    if (!fits && p.tune == 0 && !fixed) return f16_prepare_as(ctx, p, a, out, true);
+    if (!fits && p.tune == 0 && !fixed) return f16_prepare_as(ctx, p_in, a, out, true);
     if (!fits) return fail(CLDNN_B200_OUT_OF_RESOURCES, "conv_f16_tc: not enough shared memory");
     int stages = (int)((max_smem - 1024 - aux_bytes - staging_total - resident) / stage_bytes);
     if (stages > f16tc::kMaxStages) stages = f16tc::kMaxStages;
@@ -704,14 +714,14 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     void* in_ptr = (char*)const_cast<void*>(a->input0) + p.in.offset * 2;
     CUresult cr;
     if (pl.a_mode == f16tc::A_FLAT) {
-        cuuint64_t dims[2] = {(cuuint64_t)cs, (cuuint64_t)P.M_total};
+        cuuint64_t dims[2] = {a_features, (cuuint64_t)P.M_total};
         cuuint64_t strides[1] = {(cuuint64_t)(p.in.px * 2)};
         cuuint32_t box[2] = {(cuuint32_t)bke, (cuuint32_t)f16tc::kBM};
         cuuint32_t es[2] = {1, 1};
         cr = h_encode_tiled(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     } else if (pl.a_mode == f16tc::A_IM2COL) {
-        cuuint64_t dims[4] = {(cuuint64_t)cs, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
+        cuuint64_t dims[4] = {a_features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
         cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * 2), (cuuint64_t)(p.in.py * 2), (cuuint64_t)(p.in.pb * 2)};
         int lower[2] = {-p.pad_x, -p.pad_y};
         int upper[2] = {p.pad_x - (p.kw - 1) * p.dil_x, p.pad_y - (p.kh - 1) * p.dil_y};
@@ -719,7 +729,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
         cr = h_encode_im2col(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in_ptr, dims, strides, lower, upper, (cuuint32_t)bke, (cuuint32_t)f16tc::kBM, es,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     } else if (patch) {
-        cuuint64_t dims[4] = {(cuuint64_t)cs, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
+        cuuint64_t dims[4] = {a_features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
         cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * 2), (cuuint64_t)(p.in.py * 2), (cuuint64_t)(p.in.pb * 2)};
         cuuint32_t box[4] = {(cuuint32_t)bke, (cuuint32_t)pl.bw, (cuuint32_t)(pl.bh + p.kh - 1), 1};
         cuuint32_t es[4] = {1, 1, 1, 1};
@@ -728,7 +738,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     } else {
         const int sx = p.stride_x, sy = p.stride_y;
         const bool strided_view = sx != 1 || sy != 1;
-        cuuint64_t dims[4] = {(cuuint64_t)cs, (cuuint64_t)(strided_view ? P.Q : p.in.x), (cuuint64_t)(strided_view ? P.P : p.in.y), (cuuint64_t)p.in.b};
+        cuuint64_t dims[4] = {a_features, (cuuint64_t)(strided_view ? P.Q : p.in.x), (cuuint64_t)(strided_view ? P.P : p.in.y), (cuuint64_t)p.in.b};
         cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * sx * 2), (cuuint64_t)(p.in.py * sy * 2), (cuuint64_t)(p.in.pb * 2)};
         cuuint32_t box[4] = {(cuuint32_t)bke, (cuuint32_t)pl.bw, (cuuint32_t)pl.bh, (cuuint32_t)pl.bb};
         cuuint32_t es[4] = {1, 1, 1, 1};

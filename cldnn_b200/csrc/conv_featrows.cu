@@ -39,6 +39,7 @@ struct alignas(64) FrParams {
     int32_t stages, a_stage_bytes, b_stage_bytes, tx_bytes, ring_bytes;
     uint32_t sbo, layout_type, idesc, tmem_cols;
     int32_t ofm;
+    int32_t group_tiles, group_ch;            // grouped: feature tiles per group (0: one group), its input features
     int64_t out_px, out_py, out_pb, out_off, el_px, el_py, el_pb, el_off;
     int32_t el_sx, el_sy;
     void* out; const void* eltw; const void* bias; const float* quant; const float* calib; const float* ecal;
@@ -175,6 +176,7 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
             const int tw = n_tile % P.tiles_w, t2 = n_tile / P.tiles_w;
             c_w = tw * P.bw - P.pad_x; c_h = (t2 % P.tiles_h) * P.bh - P.pad_y; c_n = (t2 / P.tiles_h) * P.bb;
         }
+        const int g0 = P.group_tiles ? m_tile / P.group_tiles * P.group_ch : 0;
         int r = tap / P.kw, s = tap - r * P.kw;
         int issued = pre; bool ok = true;
         for (int i = 0; i < steps; ++i) {
@@ -186,9 +188,9 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
             }
             if (leader) {
                 const uint32_t full = smem_u32(&aux->full[st]), dst = b_base + (uint32_t)st * (uint32_t)P.b_stage_bytes;
-                if (P.mode == FR_FLAT) tma_load_2d(dst, &P.tmX, full, cc * bke, n_tile * P.cols);
-                else if (P.mode == FR_IM2COL) tma_load_im2col_4d(dst, &P.tmX, full, cc * bke, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
-                else tma_load_4d(dst, &P.tmX, full, cc * bke, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
+                if (P.mode == FR_FLAT) tma_load_2d(dst, &P.tmX, full, g0 + cc * bke, n_tile * P.cols);
+                else if (P.mode == FR_IM2COL) tma_load_im2col_4d(dst, &P.tmX, full, g0 + cc * bke, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
+                else tma_load_4d(dst, &P.tmX, full, g0 + cc * bke, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
             }
             if (++cc == P.chunks) { cc = 0; ++tap; if (++s == P.kw) { s = 0; ++r; } }
         }
@@ -348,7 +350,7 @@ bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::stri
     if (!f16 && !(p.quantization || p.calibration || p.has_o_qf)) return no("the feature-row form needs the quantised epilogue");
     if (f16 && (p.out.px % 4 || p.out.py % 4 || p.out.pb % 4 || p.out.offset % 4)) return no("the feature-row form stores four features at a time");
     pl.cols = kCols[variant / kFrSplits]; pl.split = 1 << (variant % kFrSplits);
-    const int64_t es = f16 ? 2 : 1, cs = p.in.px * es;
+    const int64_t es = f16 ? 2 : 1, cs = reduction_features(p) * es;
     const int bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32);
     const int64_t steps = (int64_t)p.kh * p.kw * (cs / bk);
     if (pl.split > steps) return no("fewer reduction steps than CTAs");
@@ -376,7 +378,7 @@ bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::stri
 // at 1024 images: 31 against 51); at a split of 2 the two are even (30 against 29 at 512 images) or this form is ahead.
 int fr_inner_product_variant(const cldnn_b200_conv_params& p)
 {
-    if (p.kh != 1 || p.kw != 1 || p.in.x != 1 || p.in.y != 1 || p.pad_x || p.pad_y || p.stride_x != 1 || p.stride_y != 1) return -1;
+    if (p.groups != 1 || p.kh != 1 || p.kw != 1 || p.in.x != 1 || p.in.y != 1 || p.pad_x || p.pad_y || p.stride_x != 1 || p.stride_y != 1) return -1;
     constexpr int64_t kSMs = 148;
     const int64_t cs = p.in.px * (p.in.dtype == CLDNN_B200_F16 ? 2 : 1), n = p.out.b, m_tiles = (p.ofm + kRows - 1) / kRows;
     const int64_t steps = cs / (cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32));
@@ -401,7 +403,7 @@ double fr_cost(const cldnn_b200_conv_params& p, int& variant)
     constexpr Cost kI8 = {4.89, 0.351, 0.00031, 0.0064, 0.0766, 0.0132, 0.893, 0.44}, kF16 = {4.09, 0.338, 0.00039, 0.0061, 0.0844, 0.0072, 1.37, 0.30};
     const bool f16 = p.in.dtype == CLDNN_B200_F16;
     const Cost& c = f16 ? kF16 : kI8;
-    const int64_t cs = p.in.px * (f16 ? 2 : 1), pixels = (int64_t)p.out.b * p.out.y * p.out.x;
+    const int64_t cs = reduction_features(p) * (f16 ? 2 : 1), pixels = (int64_t)p.out.b * p.out.y * p.out.x;
     const int64_t bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32), steps = (int64_t)p.kh * p.kw * (cs / bk), m_tiles = (p.ofm + kRows - 1) / kRows;
     double best = 0.0;
     for (int v = 0; v < kFrVariants; ++v) {
@@ -426,7 +428,7 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     FrParams P{};
     P.mode = pl.mode; P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;
     P.kw = p.kw; P.stride_x = p.stride_x; P.stride_y = p.stride_y; P.pad_x = p.pad_x; P.pad_y = p.pad_y; P.dil_x = p.dil_x; P.dil_y = p.dil_y;
-    const int64_t cs = p.in.px * es;                                 // bytes of K per tap
+    const int64_t cs = reduction_features(p) * es, xs = p.in.px * es;   // bytes of K per tap, pixel pitch of the activations
     P.bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32);
     P.chunks = (int)(cs / P.bk); P.k_steps = p.kh * p.kw * P.chunks; P.split = pl.split;
     P.cols = pl.cols; P.bw = pl.bw; P.bh = pl.bh; P.bb = pl.bb;
@@ -451,6 +453,7 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     P.idesc |= ((uint32_t)(P.cols >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
     P.tmem_cols = (uint32_t)(P.cols < 32 ? 32 : P.cols);
     P.ofm = p.ofm;
+    if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / kRows; P.group_ch = p.ifm; }
     const cldnn_b200_tensor& et = p.in_out_opt ? p.out : p.eltw;
     P.out_px = p.out.px; P.out_py = p.out.py; P.out_pb = p.out.pb; P.out_off = p.out.offset;
     if (p.fused_eltw) {
@@ -484,12 +487,12 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     void* in_ptr = (char*)const_cast<void*>(a->input0) + p.in.offset * es;
     CUresult cr;
     if (pl.mode == FR_FLAT) {
-        cuuint64_t dims[2] = {(cuuint64_t)p.in.px, (cuuint64_t)P.M_total}; cuuint64_t strides[1] = {(cuuint64_t)cs};
+        cuuint64_t dims[2] = {(cuuint64_t)p.in.px, (cuuint64_t)P.M_total}; cuuint64_t strides[1] = {(cuuint64_t)xs};
         cuuint32_t box[2] = {bke, (cuuint32_t)P.cols}; cuuint32_t one[2] = {1, 1};
         cr = fr_encode_tiled(&P.tmX, dt, 2, in_ptr, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     } else if (pl.mode == FR_IM2COL) {
         cuuint64_t dims[4] = {(cuuint64_t)p.in.px, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
-        cuuint64_t strides[3] = {(cuuint64_t)cs, (cuuint64_t)(p.in.py * es), (cuuint64_t)(p.in.pb * es)};
+        cuuint64_t strides[3] = {(cuuint64_t)xs, (cuuint64_t)(p.in.py * es), (cuuint64_t)(p.in.pb * es)};
         int lower[2] = {-p.pad_x, -p.pad_y};
         int upper[2] = {p.pad_x - (p.kw - 1) * p.dil_x, p.pad_y - (p.kh - 1) * p.dil_y};
         // the box of base pixels must produce exactly Q x P positions per image
@@ -502,13 +505,13 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
         const int sx = p.stride_x, sy = p.stride_y;                  // a pointwise strided convolution reads a strided view of the input
         const bool view = sx != 1 || sy != 1;
         cuuint64_t dims[4] = {(cuuint64_t)p.in.px, (cuuint64_t)(view ? P.Q : p.in.x), (cuuint64_t)(view ? P.P : p.in.y), (cuuint64_t)p.in.b};
-        cuuint64_t strides[3] = {(cuuint64_t)(cs * sx), (cuuint64_t)(p.in.py * sy * es), (cuuint64_t)(p.in.pb * es)};
+        cuuint64_t strides[3] = {(cuuint64_t)(xs * sx), (cuuint64_t)(p.in.py * sy * es), (cuuint64_t)(p.in.pb * es)};
         cuuint32_t box[4] = {bke, (cuuint32_t)pl.bw, (cuuint32_t)pl.bh, (cuuint32_t)pl.bb}; cuuint32_t one[4] = {1, 1, 1, 1};
         cr = fr_encode_tiled(&P.tmX, dt, 4, in_ptr, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (cr != CUDA_SUCCESS) return fail(CLDNN_B200_DEVICE_ERROR, "conv_featrows: activation tensor map rejected by the driver (CUresult " + std::to_string((int)cr) + ")");
     {
-        cuuint64_t dims[3] = {(cuuint64_t)p.in.px, (cuuint64_t)(p.kh * p.kw), (cuuint64_t)p.ofm};
+        cuuint64_t dims[3] = {(cuuint64_t)p.w_px, (cuuint64_t)(p.kh * p.kw), (cuuint64_t)p.ofm};
         cuuint64_t strides[2] = {(cuuint64_t)(p.w_px * es), (cuuint64_t)(p.w_po * es)};
         cuuint32_t box[3] = {bke, 1, (cuuint32_t)kRows}; cuuint32_t one[3] = {1, 1, 1};
         cr = fr_encode_tiled(&P.tmW, dt, 3, (char*)const_cast<void*>(a->weights) + p.w_offset * es, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,

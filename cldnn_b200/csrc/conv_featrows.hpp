@@ -6,6 +6,23 @@
 
 namespace b200 {
 
+// A convolution in groups as the tensor-core kernels see it: every feature tile of 128 lies inside one group and reads that group's
+// slice of the input features (a channel offset of the activation copies), with weights that hold the group's features only, zero
+// padded to whole chunks of the reduction.  A chunk that reaches past the slice meets the padding's zeros.  `p` comes in with feature
+// counts per group and leaves with all output features in `ofm`; `ifm` stays the reduction's.
+inline bool grouped_view(cldnn_b200_conv_params& p, std::string* why)
+{
+    auto no = [&](const char* m) { if (why) *why = m; return false; };
+    if (p.groups == 1) return true;
+    const int64_t es = p.in.dtype == CLDNN_B200_F16 ? 2 : 1;
+    if (p.groups < 1 || p.fused_eltw) return no("grouped convolution: no fused residual");
+    if (p.ofm < 128 || p.ofm % 128 || p.ifm * es % 16) return no("grouped convolution: whole feature tiles of 128 and 16-byte slices per group");
+    if (p.w_px * es % 32 || p.w_px < p.ifm || p.w_px * es >= p.ifm * es + 128) return no("grouped convolution: weights must hold one group's features, padded to whole chunks");
+    p.ofm *= p.groups;
+    return true;
+}
+inline int64_t reduction_features(const cldnn_b200_conv_params& p) { return p.groups == 1 ? p.in.px : p.w_px; }   // stored, per tap
+
 struct FrPlan {
     int mode;                                // 0 flat, 1 TMA im2col, 2 tiled box (over pixels)
     int cols, split;                         // pixel columns per tile, CTAs that share a tile's reduction

@@ -174,12 +174,12 @@ conv_i8_tc_kernel(const __grid_constant__ TcParams P)
                     const uint32_t full = smem_u32(&aux->full[stage]);
                     const uint32_t a_dst = a_base + (uint32_t)(stage * P.a_stage_bytes);
                     const uint32_t b_dst = b_base + (uint32_t)(stage * P.b_stage_bytes);
-                    const int c0 = cc * P.bk;
+                    const int c0 = cc * P.bk, a0 = c0 + (P.group_tiles ? n_tile / P.group_tiles * P.group_ch : 0);
                     if (leader) {
                         mbar_expect_tx(full, (uint32_t)(P.a_tx_bytes + P.b_tx_bytes));
-                        if (P.a_mode == A_FLAT) tma_load_2d(a_dst, &P.tmA, full, c0, m_tile * kBM);
-                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d(a_dst, &P.tmA, full, c0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
-                        else tma_load_4d(a_dst, &P.tmA, full, c0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
+                        if (P.a_mode == A_FLAT) tma_load_2d(a_dst, &P.tmA, full, a0, m_tile * kBM);
+                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d(a_dst, &P.tmA, full, a0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
+                        else tma_load_4d(a_dst, &P.tmA, full, a0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
                         tma_load_3d(b_dst, &P.tmB, full, c0, tap, n_tile * P.bn);
                     }
                     ++issued;
@@ -466,7 +466,7 @@ static void choose_patch(int Q, int Pn, int kh, int kw, int& tw, int& th)
 // conv_tile_cost.hpp; -1 in `fr_variant` unless the feature-row form is the cheapest.
 static void choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int& bn, int& groups, int& pair, int& fr_variant)
 {
-    const int64_t cs = p.in.px, pixels = (int64_t)p.out.b * p.out.y * p.out.x;
+    const int64_t cs = reduction_features(p), pixels = (int64_t)p.out.b * p.out.y * p.out.x;
     int64_t m_tiles = (pixels + kBM - 1) / kBM;
     if (mode == A_TILED) {
         int bw, bh, bb; choose_box(p.out.x, p.out.y, p.out.b, bw, bh, bb);
@@ -481,7 +481,7 @@ static void choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int&
     }
     double best = 0.0; bn = 0;
     for (int b : {64, 128, 256}) {
-        if (b > 64 && b / 2 >= p.ofm) continue;
+        if (p.groups > 1 ? b != 128 : (b > 64 && b / 2 >= p.ofm)) continue;      // (a grouped tile lies inside its group)
         const bool half_steps = b == 256 && p.fused_eltw && bk == 128 && cs < 512;     // as tc_plan sets the stage size
         const int kb = half_steps ? 64 : bk;
         const int64_t steps = (int64_t)p.kh * p.kw * (cs / kb);
@@ -497,22 +497,23 @@ static void choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int&
 }
 
 // `fixed`: the untuned choice is the one that suits every epilogue (the specialised kernel turned out not to take the launch)
-static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* why, bool fixed = false)
+static bool tc_plan(const cldnn_b200_conv_params& p_in, TcPlan& pl, std::string* why, bool fixed = false)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
+    cldnn_b200_conv_params p = p_in;
+    if (!grouped_view(p, why)) return false;
     if (!is_int8(p.in.dtype)) return no("activations must be u8 or i8");
     if (p.w_dtype != CLDNN_B200_I8) return no("weights must be i8");
-    if (p.groups != 1) return no("grouped convolution is handled by other kernels");
     if (!epilogue_order_ok(p)) return no("the MMAD / IMAD epilogue orders need quantisation, an f32 bias and an 8-bit output (IMAD fused: eltwise calibration)");
     if (p.kh < 1 || p.kw < 1 || p.kh * p.kw > 255) return no("filter size");
     if (p.stride_x < 1 || p.stride_y < 1 || p.dil_x < 1 || p.dil_y < 1) return no("stride/dilation");
-    if (p.out.f != p.ofm || p.in.f != p.ifm) return no("feature counts");
+    if (p.out.f != p.ofm || p.in.f != p.ifm * p.groups) return no("feature counts");
     if (!dense_byxf(p.in)) return no("input must be byxf with 16-byte aligned pitches");
     if (p.in.px % 32) return no("stored input features must be a multiple of 32");
     if (p.out.pf != 1) return no("output must be byxf");
     if (!(is_int8(p.out.dtype) || p.out.dtype == CLDNN_B200_F32 || p.out.dtype == CLDNN_B200_F16 || p.out.dtype == CLDNN_B200_I32)) return no("output type");
     if (p.w_pi != 1 || p.w_px % 16 || p.w_po % 16 || p.w_offset % 16 || p.w_py != p.w_px * p.kw) return no("weights must be oyxi with 16-byte aligned pitches");
-    if (p.w_px != p.in.px) return no("weights and input must store the same (padded) feature count");
+    if (p.groups == 1 && p.w_px != p.in.px) return no("weights and input must store the same (padded) feature count");
     const bool quant_path = p.quantization || p.calibration || p.has_o_qf;
     if (!quant_path && !p.fused_eltw) return no("non-quantised 8-bit convolution accumulates in 8 bits; handled by conv_ref");
     if (p.fused_eltw && !p.in_out_opt && p.eltw.pf != 1) return no("residual must be byxf");
@@ -524,7 +525,7 @@ static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* wh
     if (p.out.y != P_ || p.out.x != Q_ || p.out.b != p.in.b) return no("output size does not match the sliding-window rule");
     if ((int64_t)p.out.b * p.out.y * p.out.x > (int64_t)1 << 31) return no("too many output pixels");
 
-    const int cs = (int)p.in.px;                                    // stored channels = bytes of K per tap
+    const int cs = (int)reduction_features(p);                      // stored channels = bytes of K per tap
     pl.bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32);
     const bool is_1x1_s1 = p.kh == 1 && p.kw == 1 && p.stride_x == 1 && p.stride_y == 1 && p.pad_x == 0 && p.pad_y == 0 && pixel_dense(p.in);
     const bool pointwise = p.kh == 1 && p.kw == 1 && p.pad_x == 0 && p.pad_y == 0;
@@ -564,6 +565,7 @@ static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* wh
     // patch mode: stride-1 undilated filters whose weights fit in shared memory, specialised epilogue configuration
     auto patch_why = [&](int fbn) -> const char* {
         if (p.stride_x != 1 || p.stride_y != 1 || p.dil_x != 1 || p.dil_y != 1 || p.kh * p.kw == 1) return "patch mode needs a stride-1 undilated filter larger than 1x1";
+        if (p.groups > 1) return "patch mode reads all input features";
         if (fbn < 64 || p.ofm % fbn) return "patch mode needs output features in whole tiles of 64, 128 or 256";
         if ((size_t)p.kh * p.kw * cs * p.ofm > kPatchWeightBytes) return "patch mode keeps all weights in shared memory: at most 72 KiB";
         if (!lean_params(p)) return "patch mode exists for the specialised epilogue configuration only";
@@ -588,6 +590,8 @@ static bool tc_plan(const cldnn_b200_conv_params& p, TcPlan& pl, std::string* wh
     if (mode == A_FLAT && !is_1x1_s1) return no("flat addressing needs a dense 1x1 stride-1 convolution");
     if (mode == A_TILED && !tiled_ok) return no("tiled addressing needs stride 1 or a pointwise filter");
     if (mode == A_IM2COL && !im2col_ok) return no("im2col addressing limits exceeded (or tensor below 128 KiB)");
+    if (p.groups > 1 && bn == 0) bn = 128;
+    if (p.groups > 1 && p.ofm / p.groups % bn) return no("grouped convolution: a feature tile must lie inside one group");
     if (bn == 0) bn = p.ofm > 128 ? 256 : (p.ofm > 64 ? 128 : (p.ofm > 32 ? 64 : 32));
     if (!groups_fit(bn)) return no("four epilogue groups need feature tiles of 64 or 128 (eight or four accumulators)");
     if (mode == A_PATCH) { if (const char* m = patch_why(bn)) return no(m); }
@@ -627,10 +631,12 @@ static CUresult encode_pixel_map(CUtensorMap* tm, const TcPlan& pl, void* ptr, c
                           CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out, bool fixed)
+static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p_in, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out, bool fixed)
 {
     TcPlan pl; std::string why;
-    if (!tc_plan(p, pl, &why, fixed)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: " + why);
+    if (!tc_plan(p_in, pl, &why, fixed)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: " + why);
+    cldnn_b200_conv_params p = p_in;
+    grouped_view(p, nullptr);
     if (!a->input0 || !a->output || !a->weights) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: input, output and weights are required");
     if (p.bias_dtype != CLDNN_B200_NONE && !a->bias) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: bias_dtype set but no bias pointer");
     if (p.quantization && !a->weights_quantization_factors) return fail(CLDNN_B200_INVALID_ARG, "conv_i8_tc: quantization set but no factors");
@@ -642,13 +648,14 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
 
     if (pl.featrows) {
         const int32_t st = fr_prepare(ctx, p, a, pl.fr, out);
-        return st != CLDNN_B200_SUCCESS && p.tune == 0 && !fixed ? tc_prepare_as(ctx, p, a, out, true) : st;
+        return st != CLDNN_B200_SUCCESS && p.tune == 0 && !fixed ? tc_prepare_as(ctx, p_in, a, out, true) : st;
     }
     TcParams P{};
     P.a_mode = pl.a_mode;
     P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;
     P.kh = p.kh; P.kw = p.kw; P.stride_x = p.stride_x; P.stride_y = p.stride_y; P.pad_x = p.pad_x; P.pad_y = p.pad_y; P.dil_x = p.dil_x; P.dil_y = p.dil_y;
-    const int cs = (int)p.in.px;
+    const int cs = (int)reduction_features(p);
+    const cuuint64_t a_features = (cuuint64_t)p.in.px;               // of the activations' tensor map
     P.bk = pl.bk; P.chunks = cs / pl.bk; P.k_steps = p.kh * p.kw * P.chunks;
     P.bn = pl.bn; P.n_tiles = (p.ofm + pl.bn - 1) / pl.bn;
     P.M_total = (int64_t)P.N * P.P * P.Q;
@@ -688,6 +695,7 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
     P.nbuf = pl.bn >= 256 ? 2 : (pl.bn >= 128 ? 4 : 8);         // accumulator and staging buffers in flight: all of tensor memory
     P.tmem_cols = (uint32_t)(P.nbuf * pl.bn < 32 ? 32 : P.nbuf * pl.bn);
     P.ofm = p.ofm;
+    if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / pl.bn; P.group_ch = p.ifm; }
     P.out_px = p.out.px; P.out_py = p.out.py; P.out_pb = p.out.pb; P.out_off = p.out.offset;
     const cldnn_b200_tensor& et = p.in_out_opt ? p.out : p.eltw;
     const int esx = p.in_out_opt ? 1 : p.eltw_stride_x, esy = p.in_out_opt ? 1 : p.eltw_stride_y;
@@ -725,7 +733,7 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
     P.acc_bound = (float)p.kh * (float)p.kw * (float)p.ifm * (p.in.dtype == CLDNN_B200_U8 ? 255.0f : 128.0f) * 128.0f;
     P.epi_groups = pl.epi_groups;
     const bool use_fast = (p.tune <= 12 || p.tune > 24) && tc_fast_eligible(P);
-    if (!use_fast && p.tune == 0 && !fixed && pl.a_mode != A_PATCH) return tc_prepare_as(ctx, p, a, out, true);
+    if (!use_fast && p.tune == 0 && !fixed && pl.a_mode != A_PATCH) return tc_prepare_as(ctx, p_in, a, out, true);
     if (pl.pair && !use_fast) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: CTA pairs exist on the specialised kernel only");
     if (pl.epi_groups > 2 && !use_fast) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "conv_i8_tc: four epilogue groups exist on the specialised kernel only");
 
@@ -781,14 +789,14 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
     void* in_ptr = (char*)const_cast<void*>(a->input0) + p.in.offset;
     CUresult cr;
     if (pl.a_mode == A_FLAT) {
-        cuuint64_t dims[2] = {(cuuint64_t)cs, (cuuint64_t)P.M_total};
+        cuuint64_t dims[2] = {a_features, (cuuint64_t)P.M_total};
         cuuint64_t strides[1] = {(cuuint64_t)p.in.px};
         cuuint32_t box[2] = {(cuuint32_t)pl.bk, (cuuint32_t)kBM};
         cuuint32_t es[2] = {1, 1};
         cr = g_encode_tiled(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     } else if (pl.a_mode == A_IM2COL) {
-        cuuint64_t dims[4] = {(cuuint64_t)cs, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
+        cuuint64_t dims[4] = {a_features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
         cuuint64_t strides[3] = {(cuuint64_t)p.in.px, (cuuint64_t)p.in.py, (cuuint64_t)p.in.pb};
         int lower[2] = {-p.pad_x, -p.pad_y};
         int upper[2] = {p.pad_x - (p.kw - 1) * p.dil_x, p.pad_y - (p.kh - 1) * p.dil_y};
@@ -799,7 +807,7 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
         cr = g_encode_im2col(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, in_ptr, dims, strides, lower, upper, (cuuint32_t)pl.bk, (cuuint32_t)kBM, es,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     } else if (pl.a_mode == A_PATCH) {
-        cuuint64_t dims[4] = {(cuuint64_t)cs, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
+        cuuint64_t dims[4] = {a_features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
         cuuint64_t strides[3] = {(cuuint64_t)p.in.px, (cuuint64_t)p.in.py, (cuuint64_t)p.in.pb};
         cuuint32_t box[4] = {(cuuint32_t)pl.bk, (cuuint32_t)pl.bw, (cuuint32_t)(pl.bh + p.kh - 1), 1};
         cuuint32_t es[4] = {1, 1, 1, 1};
@@ -809,7 +817,7 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
         // tiled 4-D box; a pointwise strided convolution reads a strided view of the input
         const int sx = p.stride_x, sy = p.stride_y;
         const bool strided_view = sx != 1 || sy != 1;
-        cuuint64_t dims[4] = {(cuuint64_t)cs, (cuuint64_t)(strided_view ? P.Q : p.in.x), (cuuint64_t)(strided_view ? P.P : p.in.y), (cuuint64_t)p.in.b};
+        cuuint64_t dims[4] = {a_features, (cuuint64_t)(strided_view ? P.Q : p.in.x), (cuuint64_t)(strided_view ? P.P : p.in.y), (cuuint64_t)p.in.b};
         cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * sx), (cuuint64_t)(p.in.py * sy), (cuuint64_t)p.in.pb};
         cuuint32_t box[4] = {(cuuint32_t)pl.bk, (cuuint32_t)pl.bw, (cuuint32_t)pl.bh, (cuuint32_t)pl.bb};
         cuuint32_t es[4] = {1, 1, 1, 1};

@@ -36,6 +36,7 @@ struct alignas(64) TcParams {
     int32_t stages, a_stage_bytes, b_stage_bytes, a_tx_bytes, b_tx_bytes;
     uint32_t sbo, layout_type, idesc, tmem_cols;
     int32_t ofm;
+    int32_t group_tiles, group_ch;       // grouped: feature tiles per group (0: one group), its input features
     // epilogue
     int32_t staged;                      // 1: shared-memory tile + TMA store, 0: direct stores
     int32_t fast_epi;                    // quantised, 8-bit output and residual, simple activations

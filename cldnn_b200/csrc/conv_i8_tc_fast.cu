@@ -354,29 +354,30 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
                 if (mode == A_IM2COL) { c_w = w.d0 * P.stride_x - P.pad_x; c_h = w.d1 * P.stride_y - P.pad_y; c_n = w.d2; }
                 else if (mode == A_TILED || patch) { c_w = w.d0 * P.bw - P.pad_x; c_h = w.d1 * P.bh - P.pad_y; c_n = w.d2 * P.bb; }
                 const int m0 = w.m_tile * kBM, n0 = w.n_tile * BN;
+                const int g0 = P.group_tiles ? w.n_tile / P.group_tiles * P.group_ch : 0;    // first input feature of the tile's group
                 int tap = 0, cc = 0, off_w = 0, off_h = 0, sx = 0;
                 for (int ks = 0; ks < k_steps; ++ks) {
                     if (!__all_sync(0xffffffffu, mbar_wait_lean(empty0 + 8u * (uint32_t)stage, phase ^ 1u, s_abort, P.status, kErrProducer))) { ok = false; break; }
                     const uint32_t full = full0 + 8u * (uint32_t)stage;
                     const uint32_t dst = a_base + (uint32_t)stage * a_stage;
-                    const int c0 = cc * bk;
+                    const int c0 = cc * bk, a0 = g0 + c0;
                     if (leader && kPair) {
                         // both CTAs' copies report to rank 0's barrier, which expects the bytes of both
                         const uint32_t full_r0 = mapa_rank(full, 0u);
                         if (rank == 0u) mbar_expect_tx(full, 2u * tx);
                         tma_load_3d_pair(b_base + (uint32_t)stage * b_stage, &P.tmB, full_r0, c0, tap, n0 + (int)rank * (BN / 2));
-                        if (mode == A_FLAT) tma_load_2d_pair(dst, &P.tmA, full_r0, c0, m0);
-                        else if (mode == A_IM2COL) tma_load_im2col_4d_pair(dst, &P.tmA, full_r0, c0, c_w, c_h, c_n, (uint16_t)off_w, (uint16_t)off_h);
-                        else tma_load_4d_pair(dst, &P.tmA, full_r0, c0, c_w + off_w, c_h + off_h, c_n);
+                        if (mode == A_FLAT) tma_load_2d_pair(dst, &P.tmA, full_r0, a0, m0);
+                        else if (mode == A_IM2COL) tma_load_im2col_4d_pair(dst, &P.tmA, full_r0, a0, c_w, c_h, c_n, (uint16_t)off_w, (uint16_t)off_h);
+                        else tma_load_4d_pair(dst, &P.tmA, full_r0, a0, c_w + off_w, c_h + off_h, c_n);
                     } else if (leader) {
                         mbar_expect_tx(full, tx);
                         if (!resb) tma_load_3d(b_base + (uint32_t)stage * b_stage, &P.tmB, full, c0, tap, n0);
                         if (patch) {                                                            // one patch per filter column
                             for (int s = 0; s < kw; ++s) tma_load_4d(dst + (uint32_t)(s * patch_alloc), &P.tmA, full, c0, c_w + s, c_h, c_n);
                         }
-                        else if (mode == A_FLAT) tma_load_2d(dst, &P.tmA, full, c0, m0);
-                        else if (mode == A_IM2COL) tma_load_im2col_4d(dst, &P.tmA, full, c0, c_w, c_h, c_n, (uint16_t)off_w, (uint16_t)off_h);
-                        else tma_load_4d(dst, &P.tmA, full, c0, c_w + off_w, c_h + off_h, c_n);
+                        else if (mode == A_FLAT) tma_load_2d(dst, &P.tmA, full, a0, m0);
+                        else if (mode == A_IM2COL) tma_load_im2col_4d(dst, &P.tmA, full, a0, c_w, c_h, c_n, (uint16_t)off_w, (uint16_t)off_h);
+                        else tma_load_4d(dst, &P.tmA, full, a0, c_w + off_w, c_h + off_h, c_n);
                     }
                     ++issued;
                     if (++cc == chunks) { cc = 0; ++tap; off_w += dil_x; if (++sx == kw) { sx = 0; off_w = 0; off_h += dil_y; } }

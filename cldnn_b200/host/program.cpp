@@ -972,14 +972,25 @@ void network_impl::prepare_kernel(node* n)
         const char* tc_kernel = half_tc ? "conv_f16_tc" : "conv_i8_tc";
         if (try_tc) {
             cldnn_b200_conv_params tp = cp;
-            if (dense_groups) { tp.ofm = cp.ofm * cp.groups; tp.ifm = cp.ifm * cp.groups; tp.groups = 1; }
-            n->packed_weights = pack_conv_weights(n, stored_ifm, dense_groups ? cp.groups : 1);
-            const cldnn_b200_tensor pd = n->packed_weights.get_layout().desc();
-            tp.w_po = pd.pb; tp.w_pi = 1; tp.w_py = pd.py; tp.w_px = pd.px; tp.w_offset = 0;
-            if (fc) tp.w_px = tp.w_py = pd.pb;                         // one tap holding the whole flattened row
-            cldnn_b200_args ta = a; ta.weights = n->packed_weights.device_ptr();
             int32_t yes = 0;
-            if (cldnn_b200_kernel_supports(eng->kernel(tc_kernel), &tp, sizeof(tp), &yes) == CLDNN_B200_SUCCESS && yes) {
+            // group by group where whole feature tiles lie inside a group (weights of one group's features, padded to whole chunks of
+            // the reduction); else dense on block-diagonal weights
+            auto with_weights = [&](int32_t stored, int32_t groups) {
+                n->packed_weights = pack_conv_weights(n, stored, groups);
+                const cldnn_b200_tensor pd = n->packed_weights.get_layout().desc();
+                tp.w_po = pd.pb; tp.w_pi = 1; tp.w_py = pd.py; tp.w_px = pd.px; tp.w_offset = 0;
+                if (fc) tp.w_px = tp.w_py = pd.pb;                     // one tap holding the whole flattened row
+                yes = 0;
+                return cldnn_b200_kernel_supports(eng->kernel(tc_kernel), &tp, sizeof(tp), &yes) == CLDNN_B200_SUCCESS && yes;
+            };
+            const int32_t es = half_tc ? 2 : 1, chunk = cp.ifm * es <= 64 ? 64 : 128;
+            bool taken = dense_groups && cp.ofm % 128 == 0 && with_weights((cp.ifm * es + chunk - 1) / chunk * chunk / es, 1);
+            if (!taken) {
+                if (dense_groups) { tp.ofm = cp.ofm * cp.groups; tp.ifm = cp.ifm * cp.groups; tp.groups = 1; }
+                taken = with_weights(stored_ifm, dense_groups ? cp.groups : 1);
+            }
+            cldnn_b200_args ta = a; ta.weights = n->packed_weights.device_ptr();
+            if (taken) {
                 a = ta; cp = tp;
                 // Winograd F(2x2, 3x3) beside the direct form, behind a gate modelled on should_use_winograd_2x3_s1
                 // (src/layout_optimizer.cpp:34-53): 3x3 stride-1 undilated ungrouped fp16 convolutions whose feature counts are
