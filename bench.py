@@ -35,7 +35,7 @@ CONFIGS = {
     "alexnet_fp16": ("alexnet_fp16", 256, "AlexNet fp16 images/s", "f16", 8),
     "vgg16_fp16": ("vgg16_fp16", 32, "VGG16 fp16 images/s", "f16", 1),
 }
-HBM_KERNELS = ("conv_i8_first", "conv_first_tc", "conv_i8_dw", "pooling_i8_byxf", "pooling_f16_byxf", "pooling_ref", "lrn_f16_byxf", "lrn_ref",
+HBM_KERNELS = ("conv_i8_first", "conv_first_tc", "conv_i8_dw", "pooling_i8_byxf", "pooling_f16_byxf", "pooling_ref", "lrn_f16_byxf", "lrn_pool_f16_byxf", "lrn_ref",
                "softmax", "eltwise_ref", "eltwise_byxf", "reorder_ref", "activation_ref", "concatenation")
 
 

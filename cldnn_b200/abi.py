@@ -95,6 +95,10 @@ class PoolParams(C.Structure):
                 ("reserved", C.c_int32 * 4)]
 
 
+class LrnPoolParams(C.Structure):
+    _fields_ = [("pool", PoolParams), ("lrn_size", C.c_int32), ("lrn_k", C.c_float), ("lrn_alpha", C.c_float), ("lrn_beta", C.c_float)]
+
+
 class FcParams(C.Structure):
     _fields_ = [("in_", Tensor), ("out", Tensor),
                 ("w_dtype", C.c_int32),

@@ -75,6 +75,7 @@ extern const KernelDef kdef_pooling_ref;
 extern const KernelDef kdef_pooling_i8_byxf;
 extern const KernelDef kdef_pooling_f16_byxf;
 extern const KernelDef kdef_lrn_f16_byxf;
+extern const KernelDef kdef_lrn_pool_f16_byxf;
 extern const KernelDef kdef_fc_ref;
 extern const KernelDef kdef_softmax;
 extern const KernelDef kdef_eltwise_ref;

@@ -2,6 +2,7 @@
 // (reference order), softmax, eltwise, reorder, lrn and standalone activation.
 // The *_ref kernels take any layout through pitches; pooling_i8_byxf is the
 // feature-innermost fast path with 16-byte accesses per lane.
+#include <algorithm>
 #include <cuda_fp16.h>
 #include "engine.hpp"
 #include "sm100_ptx.cuh"
@@ -919,8 +920,42 @@ lrn_ref_kernel(const __grid_constant__ cldnn_b200_lrn_params p, const void* in, 
         store_sat_float(out, p.out.dtype, tidx(p.out, b, f, y, x), v * powf(acc, -p.beta));
     }
 }
-// The same for fp16 in the feature-innermost (byxf) layout, window 5: a thread owns 8 consecutive features of one pixel,
-// reads them with one 128-bit load and the two neighbours on either side with one 32-bit load each, keeps the squares
+// 8 consecutive features f0 .. f0 + 7 of one pixel (`src`) normalised over a window of 5: one 128-bit load and the two neighbours on
+// either side with one 32-bit load each.
+__device__ __forceinline__ uint4 lrn5_f16(const __half* src, int f0, int features, float scale, float k0, float beta)
+{
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+    float val[12];                                               // features f0 - 2 .. f0 + 9
+    {
+        const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { const float2 f = __half22float2(h[k]); val[2 + 2 * k] = f.x; val[3 + 2 * k] = f.y; }
+        float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);
+        if (f0 >= 2) lo = __half22float2(__ldg(reinterpret_cast<const __half2*>(src - 2)));
+        if (f0 + 8 < features) hi = __half22float2(__ldg(reinterpret_cast<const __half2*>(src + 8)));
+        if (f0 + 9 >= features) hi.y = 0.f;
+        val[0] = lo.x; val[1] = lo.y; val[10] = hi.x; val[11] = hi.y;
+    }
+    float sq[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) sq[k] = val[k] * val[k];
+    float pair[11];
+#pragma unroll
+    for (int k = 0; k < 11; ++k) pair[k] = sq[k] + sq[k + 1];
+    float r[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        // (flushing a subnormal power to zero changes nothing: times a half it rounds to a half zero)
+        const float e = -beta * __log2f(fmaf(pair[k] + pair[k + 2] + sq[k + 4], scale, k0));
+        float w; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(e));
+        r[k] = val[k + 2] * w;
+    }
+    __half2 o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[k] = __floats2half2_rn(r[2 * k], r[2 * k + 1]);
+    return *reinterpret_cast<const uint4*>(o);
+}
+// The same for fp16 in the feature-innermost (byxf) layout, window 5: a thread owns 8 consecutive features of one pixel, keeps the squares
 // in fp32 and writes 8 halves; x^-beta = exp2(-beta * log2(x)) on the special-function unit (the reference's
 // native_powr is as loosely specified).
 __global__ void __launch_bounds__(256)
@@ -933,30 +968,8 @@ lrn_f16_byxf_kernel(const __grid_constant__ cldnn_b200_lrn_params p, const __hal
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < (uint32_t)total; idx += gridDim.x * blockDim.x, it.next()) {   // < 2^31 items (host check)
         const int f8 = it.f, x = it.x, y = it.y, b = it.b;
         const int f0 = f8 * 8;
-        const __half* src = in + tidx(p.in, b, f0, y, x);
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
-        float val[12];                                               // features f0 - 2 .. f0 + 9
-        {
-            const __half2* h = reinterpret_cast<const __half2*>(&v);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) { const float2 f = __half22float2(h[k]); val[2 + 2 * k] = f.x; val[3 + 2 * k] = f.y; }
-            float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);
-            if (f0 >= 2) lo = __half22float2(__ldg(reinterpret_cast<const __half2*>(src - 2)));
-            if (f0 + 8 < p.in.f) hi = __half22float2(__ldg(reinterpret_cast<const __half2*>(src + 8)));
-            if (f0 + 9 >= p.in.f) hi.y = 0.f;
-            val[0] = lo.x; val[1] = lo.y; val[10] = hi.x; val[11] = hi.y;
-        }
-        float sq[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) sq[k] = val[k] * val[k];
-        __half2 o[4];
-#pragma unroll
-        for (int k = 0; k < 8; k += 2) {
-            const float a0 = fmaf(sq[k] + sq[k + 1] + sq[k + 2] + sq[k + 3] + sq[k + 4], scale, p.k);
-            const float a1 = fmaf(sq[k + 1] + sq[k + 2] + sq[k + 3] + sq[k + 4] + sq[k + 5], scale, p.k);
-            o[k >> 1] = __floats2half2_rn(val[k + 2] * exp2f(-p.beta * __log2f(a0)), val[k + 3] * exp2f(-p.beta * __log2f(a1)));
-        }
-        *reinterpret_cast<uint4*>(out + tidx(p.out, b, f0, y, x)) = *reinterpret_cast<const uint4*>(o);
+        const uint4 o = lrn5_f16(in + tidx(p.in, b, f0, y, x), f0, p.in.f, scale, p.k, p.beta);
+        *reinterpret_cast<uint4*>(out + tidx(p.out, b, f0, y, x)) = o;
     }
 }
 static bool lrn_f16_byxf_supports(const void* vp)
@@ -979,6 +992,85 @@ static int32_t lrn_f16_byxf_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, co
     out->fn = [p, in, o, grid](cudaStream_t s) { lrn_f16_byxf_kernel<<<grid, 256, 0, s>>>(p, in, o); return cudaGetLastError(); };
     return CLDNN_B200_SUCCESS;
 }
+
+// LRN and the 3x3 stride-2 maximum behind it in one pass (AlexNet's norm + pool): apart, the normalised map is written and read back,
+// 149 MB each way at 256 x 96 x 55 x 55.  A block normalises the input rows of a strip of output rows into shared memory, three
+// rows at a time (each pixel once: two special-function operations per value make recomputation as dear as the traffic), and pools from
+// there.  Values are rounded to half before the maximum, so the result is that of the two kernels apart, bit for bit.
+__global__ void __launch_bounds__(256)
+lrn_pool_f16_byxf_kernel(const __grid_constant__ cldnn_b200_lrn_pool_params p, const __half* __restrict__ in, __half* __restrict__ out, int strip)
+{
+    extern __shared__ uint4 s_rows[];                                // [iy % 3][x][feature / 8]
+    const cldnn_b200_tensor& ti = p.pool.in; const cldnn_b200_tensor& to = p.pool.out;
+    // a thread keeps its feature vector and steps over columns: no index arithmetic per value worth mentioning
+    const int fv = ti.f / 8, row_items = ti.x * fv, b = blockIdx.y;
+    const int f8 = threadIdx.x % fv, x0 = threadIdx.x / fv, xs = blockDim.x / fv, f0 = f8 * 8;
+    const int oy0 = blockIdx.x * strip, oy1 = min(oy0 + strip, to.y);
+    const float scale = __fdiv_rn(p.lrn_alpha, (float)p.lrn_size);
+    const __half* src = in + tidx(ti, b, f0, 0, x0);
+    __half* dst = out + tidx(to, b, f0, 0, x0);
+    for (int oy = oy0; oy < oy1; ++oy) {
+        for (int iy = oy == oy0 ? 2 * oy : 2 * oy + 1; iy < 2 * oy + 3; ++iy) {          // the row above is there from the output row before
+            const __half* row = src + (int64_t)iy * ti.py;
+            uint4* to_row = s_rows + (iy % 3) * row_items + f8;
+            if (x0 < xs)
+#pragma unroll 2
+                for (int x = x0; x < ti.x; x += xs) to_row[x * fv] = lrn5_f16(row + (int64_t)(x - x0) * ti.px, f0, ti.f, scale, p.lrn_k, p.lrn_beta);
+        }
+        __syncthreads();
+        if (x0 < xs)
+            for (int x = x0; x < to.x; x += xs) {
+                const __half2 lowest = __half2half2(__ushort_as_half((unsigned short)0xfbffu));   // as the pooling kernel starts
+                __half2 m[4] = {lowest, lowest, lowest, lowest};
+                const uint4* at = s_rows + 2 * x * fv + f8;
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+#pragma unroll
+                    for (int s = 0; s < 3; ++s) {
+                        const uint4 v = at[r * row_items + s * fv];
+                        const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) m[q] = __hmax2(m[q], h[q]);
+                    }
+                *reinterpret_cast<uint4*>(dst + (int64_t)oy * to.py + (int64_t)(x - x0) * to.px) = *reinterpret_cast<const uint4*>(m);
+            }
+        __syncthreads();
+    }
+}
+static size_t lrn_pool_smem(const cldnn_b200_lrn_pool_params& p) { return (size_t)3 * p.pool.in.x * p.pool.in.f * 2; }
+static bool lrn_pool_supports(const void* vp)
+{
+    const auto& p = *(const cldnn_b200_lrn_pool_params*)vp;
+    const cldnn_b200_pool_params& q = p.pool;
+    if (p.lrn_size != 5 || q.in.dtype != CLDNN_B200_F16 || q.out.dtype != CLDNN_B200_F16) return false;
+    if (q.mode != CLDNN_B200_POOL_MAX || q.size_x != 3 || q.size_y != 3 || q.stride_x != 2 || q.stride_y != 2 || q.pad_x || q.pad_y || q.act != CLDNN_B200_ACT_NONE) return false;
+    if (q.in.pf != 1 || q.out.pf != 1 || q.in.f % 8 || q.in.f < 8 || q.in.f > 2048 || q.in.f != q.out.f || q.in.b != q.out.b || q.in.b < 1 || q.in.b > 65535) return false;
+    if (q.out.x < 1 || q.out.y < 1 || 2 * q.out.x + 1 > q.in.x || 2 * q.out.y + 1 > q.in.y) return false;   // windows inside the map
+    const int64_t pitches[] = {q.in.px, q.in.py, q.in.pb, q.in.offset, q.out.px, q.out.py, q.out.pb, q.out.offset};
+    for (int64_t v : pitches) if (v % 8) return false;
+    return lrn_pool_smem(p) <= 64 * 1024;
+}
+static int32_t lrn_pool_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)
+{
+    const cldnn_b200_lrn_pool_params p = *(const cldnn_b200_lrn_pool_params*)vp;
+    if (!lrn_pool_supports(vp)) return fail(CLDNN_B200_UNSUPPORTED_FORMAT, "lrn_pool_f16_byxf: fp16 byxf, up to 2048 features, LRN window 5, 3x3 stride-2 maximum without padding");
+    if (!a->input0 || !a->output) return fail(CLDNN_B200_INVALID_ARG, "lrn_pool_f16_byxf: input and output are required");
+    if (((uintptr_t)a->input0 | (uintptr_t)a->output) & 15) return fail(CLDNN_B200_INVALID_ARG, "lrn_pool_f16_byxf: buffers must be 16-byte aligned");
+    const __half* in = (const __half*)a->input0; __half* o = (__half*)a->output;
+    const size_t smem = lrn_pool_smem(p);
+    B200_CUDA(raise_smem_limit((const void*)lrn_pool_f16_byxf_kernel, ctx->device, smem));
+    // the strip with the least work per wave of resident blocks: 2 * strip + 1 input rows each
+    const int64_t per_sm = std::min<int64_t>(8, (int64_t)(ctx->prop.sharedMemPerMultiprocessor / (smem + 1024))), slots = per_sm * ctx->prop.multiProcessorCount;
+    int strip = 1; int64_t best = 0;
+    for (int r = 1; r <= p.pool.out.y; ++r) {
+        const int64_t blocks = (int64_t)p.pool.out.b * ((p.pool.out.y + r - 1) / r), cost = (blocks + slots - 1) / slots * (2 * r + 1);
+        if (r == 1 || cost < best) { best = cost; strip = r; }
+    }
+    const dim3 grid((unsigned)((p.pool.out.y + strip - 1) / strip), (unsigned)p.pool.out.b);
+    out->fn = [p, in, o, grid, smem, strip](cudaStream_t s) { lrn_pool_f16_byxf_kernel<<<grid, 256, smem, s>>>(p, in, o, strip); return cudaGetLastError(); };
+    return CLDNN_B200_SUCCESS;
+}
+const KernelDef kdef_lrn_pool_f16_byxf = {"lrn_pool_f16_byxf", sizeof(cldnn_b200_lrn_pool_params), lrn_pool_supports, one_tune, nullptr, lrn_pool_prepare};
 
 static bool lrn_supports(const void* vp) { const auto& p = *(const cldnn_b200_lrn_params*)vp; return p.size >= 1 && is_fp(p.in.dtype); }
 static int32_t lrn_prepare(cldnn_b200_ctx_impl* ctx, const void* vp, const cldnn_b200_args* a, cldnn_b200_prepared_impl* out)

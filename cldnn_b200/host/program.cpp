@@ -249,6 +249,7 @@ struct node {
     // fused activations (prepare_primitive_fusing)
     int32_t act = CLDNN_B200_ACT_NONE; float act_m = 0.f, act_n = 0.f;
     int32_t eltw_act = CLDNN_B200_ACT_NONE; float eltw_m = 0.f, eltw_n = 0.f;
+    int32_t lrn_size = 0; float lrn_k = 0.f, lrn_alpha = 0.f, lrn_beta = 0.f;   // pooling: the LRN folded in front of it
     // execution
     memory mem;                         // output memory
     memory packed_weights;              // weights re-laid for the chosen kernel
@@ -312,6 +313,7 @@ public:
     void calc_layout(node* n);
     void fuse_activations();
     void fuse_conv_eltwise();
+    void fuse_lrn_pool();
     void select_layouts();
     void conv_eltw_read_write_opt();
     void replace_dep(node* consumer, node* from, node* to) { for (auto& id : consumer->p.input) if (id == from->p.id) id = to->p.id; }
@@ -448,6 +450,28 @@ void network_impl::fuse_activations()
         if (a->is_output) { prod->is_output = true; prod->answers_for = a->answers_for.empty() ? a->p.id : a->answers_for; }
         by_id[a->p.id] = prod;
         a->removed = true;
+        link();
+    }
+    sort(); relayout();
+}
+
+// LRN whose only reader is a 3x3 stride-2 maximum: one launch for both (lrn_pool_f16_byxf).
+void network_impl::fuse_lrn_pool()
+{
+    for (size_t i = 0; i < nodes.size(); ++i) {
+        node* n = nodes[i].get();
+        if (n->removed || n->p.type != "pooling" || n->deps.size() != 1 || n->lrn_size || n->act != CLDNN_B200_ACT_NONE) continue;
+        node* l = n->deps[0];
+        if (l->p.type != "lrn" || l->users.size() != 1 || l->is_output || l->deps.size() != 1 || l->deps[0]->out.data_type != data_types::f16) continue;
+        const bool window = n->p.pool_mode == pooling_mode::max && !n->p.global_pooling && n->p.size.x == 3 && n->p.size.y == 3 && n->p.stride.x == 2 &&
+                            n->p.stride.y == 2 && n->p.input_offset.x == 0 && n->p.input_offset.y == 0;
+        const tensor& ls = l->out.size; const tensor& os = n->out.size;
+        if (!window || l->p.lrn_size != 5 || ls.feature % 8 || ls.feature > 2048 || 2 * os.x + 1 > ls.x || 2 * os.y + 1 > ls.y) continue;
+        if ((size_t)3 * ls.x * ls.feature * 2 > 64 * 1024 || ls.batch > 65535) continue;          // the kernel's three rows in shared memory
+        n->lrn_size = (int32_t)l->p.lrn_size; n->lrn_k = l->p.lrn_k; n->lrn_alpha = l->p.lrn_alpha; n->lrn_beta = l->p.lrn_beta;
+        n->p.input[0] = l->deps[0]->p.id;
+        n->fused_ids += (n->fused_ids.empty() ? "" : ",") + l->p.id;
+        l->removed = true;
         link();
     }
     sort(); relayout();
@@ -1050,6 +1074,31 @@ void network_impl::prepare_kernel(node* n)
         if (p.pool_mode == pooling_mode::average && dyn) pp.div_mode = CLDNN_B200_DIV_DYNAMIC_WITH_PADDING;
         else pp.div_mode = p.pool_mode == pooling_mode::average_no_padding ? CLDNN_B200_DIV_DYNAMIC : CLDNN_B200_DIV_FIXED;
         pp.act = n->act; pp.act_m = n->act_m; pp.act_n = n->act_n;
+        if (n->lrn_size) {
+            cldnn_b200_lrn_pool_params fp{}; fp.pool = pp;
+            fp.lrn_size = n->lrn_size; fp.lrn_k = n->lrn_k; fp.lrn_alpha = n->lrn_alpha; fp.lrn_beta = n->lrn_beta;
+            int32_t yes = 0;
+            if (cldnn_b200_kernel_supports(eng->kernel("lrn_pool_f16_byxf"), &fp, sizeof(fp), &yes) == CLDNN_B200_SUCCESS && yes) {
+                finish({"lrn_pool_f16_byxf"}, &fp, sizeof(fp), [](int) {});
+                return;
+            }
+            // a layout the joint kernel does not take: the two launches, with the normalised map in a workspace
+            n->scratch = new_block(eng, in.bytes_count());
+            cldnn_b200_lrn_params lp{}; lp.in = lp.out = in.desc();
+            lp.size = n->lrn_size; lp.k = n->lrn_k; lp.alpha = n->lrn_alpha; lp.beta = n->lrn_beta;
+            cldnn_b200_args la = a; la.output = n->scratch->dev; a.input0 = n->scratch->dev;
+            auto first_of = [&](const std::vector<std::string>& cands, const void* params, size_t size) {
+                for (auto& c : cands) if (cldnn_b200_kernel_supports(eng->kernel(c), params, size, &yes) == CLDNN_B200_SUCCESS && yes) return c;
+                throw error(p.id + ": cannot find a proper kernel with these arguments", CLDNN_B200_ERROR);
+            };
+            cldnn_b200_prepared second = nullptr;
+            const std::string lk = first_of({"lrn_f16_byxf", "lrn_ref"}, &lp, sizeof(lp));
+            n->kernel = first_of({"pooling_f16_byxf", "pooling_ref"}, &pp, sizeof(pp)); n->tune = 0;
+            check(cldnn_b200_prepare(eng->kernel(lk), &lp, sizeof(lp), &la, &n->prepared), p.id + " (" + lk + ")");
+            check(cldnn_b200_prepare(eng->kernel(n->kernel), &pp, sizeof(pp), &a, &second), p.id + " (" + n->kernel + ")");
+            n->more_prepared.push_back(second);
+            return;
+        }
         finish({"pooling_i8_byxf", "pooling_f16_byxf", "pooling_ref"}, &pp, sizeof(pp), [](int) {});
         return;
     }
@@ -1175,6 +1224,7 @@ void network_impl::build(const topology& topo)
         fuse_activations();
         fuse_conv_eltwise();
         fuse_activations();                                         // relu behind a freshly fused conv+eltwise
+        fuse_lrn_pool();
         select_layouts();
         if (opts.conv_eltw_read_write_opt) conv_eltw_read_write_opt();
     }

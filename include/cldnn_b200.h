@@ -169,6 +169,12 @@ typedef struct cldnn_b200_pool_params {
     int32_t reserved[4];
 } cldnn_b200_pool_params;
 
+/* Across-channel LRN followed by pooling in one launch (lrn_pool_f16_byxf): pool.in is the LRN's input. */
+typedef struct cldnn_b200_lrn_pool_params {
+    cldnn_b200_pool_params pool;
+    int32_t lrn_size; float lrn_k, lrn_alpha, lrn_beta;
+} cldnn_b200_lrn_pool_params;
+
 /* fully_connected constants (fully_connected_gpu::create,
  * src/gpu/fully_connected_gpu.cpp:59-112; arithmetic of
  * cl_kernels/fully_connected_gpu_bfyx_ref.cl:18-84). Weights [ofm][f][y][x]. */
