@@ -191,6 +191,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
     const uint32_t tmem_base = aux->tmem_base;
     const bool patch = P.a_mode == A_PATCH;
     const bool boxed = P.a_mode == A_TILED || patch;
+    griddep_launch_dependents();
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------

@@ -200,6 +200,7 @@ conv_first_tc_kernel(const __grid_constant__ Params P)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = aux->tmem_base;
+    griddep_launch_dependents();
     const int my_tiles = (P.total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
     if (warp < kBuildWarps) {

@@ -32,6 +32,7 @@ template <bool kUnsignedIn>
 __global__ void __launch_bounds__(256)
 conv_i8_dw_kernel(const __grid_constant__ cldnn_b200_conv_params p, const __grid_constant__ EpiCfg c, DwArgs a)
 {
+    ptx::griddep_launch_dependents();
     extern __shared__ int8_t s_w[];                                  // [kh*kw][C]
     const int C = p.out.f, taps = p.kh * p.kw;
     for (int i = threadIdx.x; i < taps * C; i += blockDim.x) {
@@ -157,6 +158,7 @@ template <bool kUnsignedIn>
 __global__ void __launch_bounds__(256)
 conv_i8_dw16_kernel(const __grid_constant__ cldnn_b200_conv_params p, const __grid_constant__ EpiCfg c, const __grid_constant__ Dw16Args a)
 {
+    ptx::griddep_launch_dependents();
     extern __shared__ uint4 s_dw[];
     const int C = p.out.f, taps = p.kh * p.kw;
     uint4* s_w = s_dw;                                               // [tap][k][C / 16]: the 4 weight words of features 16 g + 4 k .. + 3 (threads of a warp differ in g: consecutive 16-byte reads)
@@ -393,6 +395,7 @@ template <bool kUnsignedIn, int kStride>
 __global__ void __launch_bounds__(256, kStride == 1 ? 3 : 2)
 conv_i8_dwcol_kernel(const __grid_constant__ cldnn_b200_conv_params p, const __grid_constant__ EpiCfg c, const __grid_constant__ Dw16Args a)
 {
+    ptx::griddep_launch_dependents();
     // the epilogue variant is uniform over the launch: chosen once, so that the row loop is straight-line code
     const bool wide = __ldg(a.wide_flag) != 0u;
     const int mode = (a.lean && !wide) ? (p.out.dtype == CLDNN_B200_U8 ? 0 : (c.act == CLDNN_B200_ACT_RELU ? 2 : 1)) : 3;

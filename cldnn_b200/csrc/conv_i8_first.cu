@@ -206,6 +206,7 @@ conv_i8_first_kernel(const __grid_constant__ FirstParams P)
     }
     if (warp == 8) { tmem_alloc(smem_u32(&aux->tmem_base), P.tmem_cols); tmem_relinquish(); }
     __syncthreads();
+    griddep_launch_dependents();
     // weights image and per-feature constants: once per CTA
     for (int i = tid; i < b_bytes / 16; i += kFThreads) reinterpret_cast<uint4*>(sB)[i] = __ldg(reinterpret_cast<const uint4*>(P.wpacked) + i);
     for (int j = tid; j < P.ofm; j += kFThreads) {

@@ -299,6 +299,7 @@ conv_i8_first_rows_kernel(const __grid_constant__ RowsParams P)
     }
     if (warp == 1) { tmem_alloc(smem_u32(&aux->tmem_base), 512u); tmem_relinquish(); }
     __syncthreads();
+    griddep_launch_dependents();
     for (int j = tid; j < P.ofm; j += kRThreads) {
         if (kHalf) { aux->bias_f[j] = P.bias_dtype != CLDNN_B200_NONE ? load_as_float(P.bias, P.bias_dtype, j) : 0.0f; continue; }
         const int32_t bi = c.bias_dtype != CLDNN_B200_NONE ? ((const int32_t*)P.bias)[j] : 0;

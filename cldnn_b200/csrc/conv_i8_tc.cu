@@ -135,6 +135,7 @@ conv_i8_tc_kernel(const __grid_constant__ TcParams P)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = aux->tmem_base;
+    griddep_launch_dependents();
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------

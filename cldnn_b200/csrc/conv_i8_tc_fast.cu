@@ -533,7 +533,6 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
         }
     } else if (warp >= kFastEpiWarp0) {
         // ------------------------------ epilogue ----------------------------------
-        griddep_wait();                                             // (it reads only constants from global memory, and the status word)
         const int ew = warp - kFastEpiWarp0;
         const int quad = ew & 3;                                    // TMEM lanes 32*quad .. 32*quad+31 (warp index mod 4)
         const int group = ew >> 2;
@@ -574,6 +573,7 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
                 if (lane == 0) aux->wide[group][quad] = w ? 1u : 0u;
                 named_bar_sync(1 + group, 128);
                 wide = (aux->wide[group][0] | aux->wide[group][1] | aux->wide[group][2] | aux->wide[group][3]) != 0u;
+                if (cur_n_tile < 0) griddep_wait();                 // (the constants above are the network's: fetched before the wait)
                 cur_n_tile = n_tile;
             }
             if (!mbar_wait(smem_u32(&aux->tmem_full[acc]), par, s_abort, P.status, kErrEpilogue)) { ok = false; break; }

@@ -174,6 +174,7 @@ template <bool kUnsignedIn>
 __global__ void __launch_bounds__(256)
 pooling_i8_byxf_kernel(const __grid_constant__ cldnn_b200_pool_params p, const uint8_t* __restrict__ in, uint8_t* __restrict__ out)
 {
+    ptx::griddep_launch_dependents();
     const int fv = p.in.f / 16;
     const int64_t total = (int64_t)p.out.b * p.out.y * p.out.x * fv;
     const bool fast_max = p.mode == CLDNN_B200_POOL_MAX && (p.act == CLDNN_B200_ACT_NONE || p.act == CLDNN_B200_ACT_RELU);
@@ -292,6 +293,7 @@ __global__ void __launch_bounds__(kWinSlices * kWinVecs)
 pooling_i8_window_kernel(const __grid_constant__ cldnn_b200_pool_params p, const uint8_t* __restrict__ in, uint8_t* __restrict__ out)
 {
     __shared__ uint32_t part[kWinSlices][kWinVecs][8];
+    ptx::griddep_launch_dependents();
     const int fv = p.in.f / 16, groups = (fv + kWinVecs - 1) / kWinVecs;
     uint32_t t = blockIdx.x;
     const int g = (int)(t % (uint32_t)groups); t /= (uint32_t)groups;
@@ -403,6 +405,7 @@ __device__ __forceinline__ void pool_max_clamped(const __half* src, int64_t px, 
 __global__ void __launch_bounds__(256)
 pooling_f16_byxf_kernel(const __grid_constant__ cldnn_b200_pool_params p, const __half* __restrict__ in, __half* __restrict__ out)
 {
+    ptx::griddep_launch_dependents();
     const int fv = p.in.f / 8;
     const int64_t total = (int64_t)p.out.b * p.out.y * p.out.x * fv;
     const bool is_max = p.mode == CLDNN_B200_POOL_MAX;
@@ -1025,6 +1028,7 @@ __device__ __forceinline__ uint4 lrn5_f16(const __half* src, int f0, int feature
 __global__ void __launch_bounds__(256)
 lrn_f16_byxf_kernel(const __grid_constant__ cldnn_b200_lrn_params p, const __half* __restrict__ in, __half* __restrict__ out)
 {
+    ptx::griddep_launch_dependents();
     const int fv = p.in.f / 8;
     const int64_t total = (int64_t)p.in.b * p.in.y * p.in.x * fv;
     const float scale = __fdiv_rn(p.alpha, (float)p.size);
@@ -1065,6 +1069,7 @@ __global__ void __launch_bounds__(256)
 lrn_pool_f16_byxf_kernel(const __grid_constant__ cldnn_b200_lrn_pool_params p, const __half* __restrict__ in, __half* __restrict__ out, int strip)
 {
     extern __shared__ uint4 s_rows[];                                // [iy % 3][x][feature / 8]
+    ptx::griddep_launch_dependents();
     const cldnn_b200_tensor& ti = p.pool.in; const cldnn_b200_tensor& to = p.pool.out;
     // a thread keeps its feature vector and steps over columns: no index arithmetic per value worth mentioning
     const int fv = ti.f / 8, row_items = ti.x * fv, b = blockIdx.y;
