@@ -63,6 +63,7 @@ struct alignas(64) Params {
     int32_t b_total_bytes, patch_alloc;      // patch mode: all taps' weights (resident), bytes reserved per patch
     int32_t batch_tiles;                     // batched GEMM view: tiles per batch, the weight 'tap' is the batch index (0 = plain convolution)
     int32_t ofm, fused, bias_dtype, act, eltw_act;
+    int32_t pair;                            // CTA pairs: m_tiles is even, the weight box holds bn / 2 rows
     int32_t group_tiles, group_ch;           // grouped: feature tiles per group (0: one group), its input features
     float act_m, act_n, eltw_m, eltw_n;
     const void* bias;
@@ -72,6 +73,7 @@ struct alignas(64) Params {
 struct Aux {
     uint64_t full[kMaxStages], empty[kMaxStages];
     uint64_t tmem_full[kMaxBufs], tmem_empty[kMaxBufs], res_full[kMaxBufs], stage_free[kMaxBufs], out_ready[kMaxBufs];
+    uint64_t drain;                          // CTA pairs: every issued instruction has retired
     uint64_t b_full;                         // patch mode: the resident weights have landed
     uint32_t tmem_base, abort;
     alignas(16) float bias[kGroups][kMaxBN];
@@ -86,12 +88,14 @@ __device__ __forceinline__ uint64_t desc64(uint32_t lo, uint32_t hi)
 {
     uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi)); return d;
 }
-template <int KK>
+template <int KK, bool kPair = false>
 __device__ __forceinline__ void mma_chunk(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t acc_first)
 {
 #pragma unroll
-    for (int k = 0; k < KK; ++k)
-        mma_f16_ss(d_tmem, desc64(a_lo + 2u * k, hi), desc64(b_lo + 2u * k, hi), idesc, k ? 1u : acc_first);
+    for (int k = 0; k < KK; ++k) {
+        if (kPair) mma_f16_ss_pair(d_tmem, desc64(a_lo + 2u * k, hi), desc64(b_lo + 2u * k, hi), idesc, k ? 1u : acc_first);
+        else mma_f16_ss(d_tmem, desc64(a_lo + 2u * k, hi), desc64(b_lo + 2u * k, hi), idesc, k ? 1u : acc_first);
+    }
 }
 
 // the activations outside NONE / ReLU stay out of line: the unrolled epilogue body would otherwise carry 64 copies
@@ -142,7 +146,11 @@ __device__ __forceinline__ void chunk_ptrs(uint8_t* stg, int row, uint32_t sw, i
     for (int w = 0; w < 4; ++w) p[w] = reinterpret_cast<uint4*>(rowp + ((((uint32_t)o >> 4) + (uint32_t)w) ^ sw) * 16u);
 }
 
-template <int BN, bool kFused>
+// kPair: the two CTAs of a cluster work on vertically adjacent pixel tiles with one instruction stream (cta_group::2, M = 256), as in the
+// 8-bit kernel: each loads its own 128 pixel rows and half of the feature tile's weight rows, every copy reports to rank 0's
+// barriers, rank 0 issues and releases stages and accumulators to both.  A stage of a 256-feature tile is 32 KiB instead of 48, so five
+// fit instead of three and an SM takes in a third fewer rows per step.
+template <int BN, bool kFused, bool kPair = false>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_f16_tc_kernel(const __grid_constant__ Params P)
 {
@@ -170,27 +178,34 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
     Aux* aux = reinterpret_cast<Aux*>(smem + (uint32_t)P.ring_bytes + (uint32_t)NSTG * kStagingBytes);
     volatile uint32_t* s_abort = &aux->abort;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = kPair ? cluster_ctarank() : 0u;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.stages; ++s) { mbar_init(smem_u32(&aux->full[s]), 1); mbar_init(smem_u32(&aux->empty[s]), 1); }
         for (int a = 0; a < kMaxBufs; ++a) {
-            mbar_init(smem_u32(&aux->tmem_full[a]), 1); mbar_init(smem_u32(&aux->tmem_empty[a]), 4);
+            mbar_init(smem_u32(&aux->tmem_full[a]), 1); mbar_init(smem_u32(&aux->tmem_empty[a]), kPair ? 8 : 4);
             mbar_init(smem_u32(&aux->res_full[a]), 1); mbar_init(smem_u32(&aux->stage_free[a]), 1);
             mbar_init(smem_u32(&aux->out_ready[a]), 4);
         }
-        mbar_init(smem_u32(&aux->b_full), 1);
+        mbar_init(smem_u32(&aux->b_full), 1); mbar_init(smem_u32(&aux->drain), 1);
         aux->abort = 0u;
         mbar_fence_init();
         prefetch_tensormap(&P.tmA); prefetch_tensormap(&P.tmB); prefetch_tensormap(&P.tmO);
         if (kFused) prefetch_tensormap(&P.tmE);
     }
-    if (warp == 1) { tmem_alloc(smem_u32(&aux->tmem_base), P.tmem_cols); tmem_relinquish(); }
+    if (warp == 1) {
+        if (kPair) { tmem_alloc_pair(smem_u32(&aux->tmem_base), P.tmem_cols); tmem_relinquish_pair(); }
+        else { tmem_alloc(smem_u32(&aux->tmem_base), P.tmem_cols); tmem_relinquish(); }
+    }
     tc_fence_before();
-    __syncthreads();
+    if (kPair) cluster_sync_all();                     // the peer's barriers exist before anything arrives on them
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = aux->tmem_base;
     const bool patch = P.a_mode == A_PATCH;
     const bool boxed = P.a_mode == A_TILED || patch;
+    // Each role waits for the previous kernel of the stream before it first touches memory that kernel wrote or read; weights are
+    // constants of the network, and the patch mode's resident copy of them starts before that.
     griddep_launch_dependents();
 
     if (warp == 0) {
@@ -209,6 +224,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
                 for (int tp = 0; tp < P.kh * P.kw; ++tp)
                     for (int ch = 0; ch < P.chunks; ++ch, dst += (uint32_t)P.b_stage_bytes) tma_load_3d(dst, &P.tmB, bf, ch * bke, tp, 0);
             }
+            griddep_wait();
             for (int tile = blockIdx.x; tile < P.total_tiles && ok; tile += gridDim.x) {
                 const int n_tile = tile / P.m_tiles, m_tile = tile - n_tile * P.m_tiles;
                 int c_w = 0, c_h = 0, c_n = 0;
@@ -231,6 +247,14 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
                     if (leader && patch) {
                         mbar_expect_tx(full, (uint32_t)P.a_tx_bytes);
                         for (int sc = 0; sc < P.kw; ++sc) tma_load_4d(a_dst + (uint32_t)(sc * P.patch_alloc), &P.tmA, full, c0, c_w + sc, c_h, c_n);
+                    } else if (leader && kPair) {
+                        // both CTAs' copies report to rank 0's barrier, which expects the bytes of both
+                        const uint32_t full_r0 = mapa_rank(full, 0u);
+                        if (rank == 0u) mbar_expect_tx(full, 2u * (uint32_t)(P.a_tx_bytes + P.b_tx_bytes));
+                        if (P.a_mode == A_FLAT) tma_load_2d_pair(a_dst, &P.tmA, full_r0, a0, m_tile * kBM);
+                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d_pair(a_dst, &P.tmA, full_r0, a0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
+                        else tma_load_4d_pair(a_dst, &P.tmA, full_r0, a0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
+                        tma_load_3d_pair(b_dst, &P.tmB, full_r0, c0, tap, n_tile * BN + (int)rank * (BN / 2));
                     } else if (leader) {
                         mbar_expect_tx(full, (uint32_t)(P.a_tx_bytes + P.b_tx_bytes));
                         if (P.a_mode == A_FLAT) tma_load_2d(a_dst, &P.tmA, full, a0, m_tile * kBM);
@@ -256,7 +280,8 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        {
+        // (in a pair only the CTA of rank 0 issues; its instructions and commits act on both CTAs)
+        if (!kPair || rank == 0u) {
             const bool leader = elect_one();
             const uint32_t hi = desc_hi(P.sbo, P.layout_type);
             const uint32_t a_lo0 = desc_lo(a_base), b_lo0 = desc_lo(b_base);
@@ -291,22 +316,31 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
                             }
                         tc_commit(empty0 + 8u * (uint32_t)stage);
                     } else if (leader) {
-                        if (kk == 4) mma_chunk<4>(d_tmem, a_lo, b_lo, hi, idesc, accf);
-                        else if (kk == 2) mma_chunk<2>(d_tmem, a_lo, b_lo, hi, idesc, accf);
-                        else mma_chunk<1>(d_tmem, a_lo, b_lo, hi, idesc, accf);
-                        tc_commit(empty0 + 8u * (uint32_t)stage);
+                        if (kk == 4) mma_chunk<4, kPair>(d_tmem, a_lo, b_lo, hi, idesc, accf);
+                        else if (kk == 2) mma_chunk<2, kPair>(d_tmem, a_lo, b_lo, hi, idesc, accf);
+                        else mma_chunk<1, kPair>(d_tmem, a_lo, b_lo, hi, idesc, accf);
+                        if (kPair) tc_commit_pair(empty0 + 8u * (uint32_t)stage); else tc_commit(empty0 + 8u * (uint32_t)stage);
                     }
                     accf = 1u;
                     if (++stage == stages) { stage = 0; phase ^= 1u; a_lo = a_lo0; b_lo = b_lo0; }
                     else { a_lo += a_step; b_lo += b_step; }
                 }
-                if (ok && leader) tc_commit(smem_u32(&aux->tmem_full[acc]));
+                if (ok && leader) { if (kPair) tc_commit_pair(smem_u32(&aux->tmem_full[acc])); else tc_commit(smem_u32(&aux->tmem_full[acc])); }
+            }
+            if (kPair) {
+                // drain: the instructions read the peer's shared memory, so every one of them retires before the pair leaves
+                if (leader) tc_commit(smem_u32(&aux->drain));
+                const uint64_t t0 = globaltimer();
+                while (!mbar_try_wait(smem_u32(&aux->drain), 0u)) {
+                    if (globaltimer() - t0 > kWaitLimitNs) { atomicCAS(P.status, 0u, kErr + 8u); break; }
+                }
             }
         }
     } else if (warp == 2) {
         // ------------------------------ TMA store issuer --------------------------
         {
             const bool leader = elect_one();                           // issues, commits and waits for the stores: bulk groups are per thread
+            griddep_wait();
             bool alive = true;
             for (int i0 = 0; alive && (int64_t)blockIdx.x + (int64_t)i0 * gridDim.x < P.total_tiles; i0 += 2) {
                 for (int h = 0; h < UNITS && alive; ++h) {
@@ -339,6 +373,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
         // ------------------------------ residual loader ---------------------------
         if (kFused) {
             const bool leader = elect_one();
+            griddep_wait();
             bool alive = true;
             for (int i0 = 0; alive && (int64_t)blockIdx.x + (int64_t)i0 * gridDim.x < P.total_tiles; i0 += 2) {
                 for (int h = 0; h < UNITS && alive; ++h) {
@@ -368,6 +403,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
         }
     } else {
         // ------------------------------ epilogue ----------------------------------
+        griddep_wait();
         const int ew = warp - kEpiWarp0;
         const int quad = ew & 3, group = ew >> 2;
         const int row = quad * 32 + lane;
@@ -404,7 +440,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
                     uint32_t r[32];
                     tmem_ld_32x32(t_row + (uint32_t)c0, r);
                     tmem_ld_wait();
-                    if (c0 + 32 >= BN) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(smem_u32(&aux->tmem_empty[acc])); }
+                    if (c0 + 32 >= BN) { tc_fence_before(); __syncwarp(); if (lane == 0) { if (kPair) mbar_arrive_cluster(mapa_rank(smem_u32(&aux->tmem_empty[acc]), 0u)); else mbar_arrive(smem_u32(&aux->tmem_empty[acc])); } }
                     if (n_tile * BN + c0 >= P.ofm) continue;
                     uint4* p[4];
                     chunk_ptrs(stg, row, sw, c0 - h * UW, p);
@@ -417,8 +453,9 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
         }
     }
     tc_fence_before();
-    __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, P.tmem_cols); }
+    if (kPair) cluster_sync_all();
+    else __syncthreads();
+    if (warp == 1) { tc_fence_after(); if (kPair) tmem_dealloc_pair(tmem_base, P.tmem_cols); else tmem_dealloc(tmem_base, P.tmem_cols); }
 }
 
 }  // namespace f16tc
@@ -452,12 +489,14 @@ static bool f16_driver_entry_points()
     return h_encode_tiled && h_encode_im2col;
 }
 
-struct F16Plan { int a_mode, bn, bk, bw, bh, bb; bool featrows; FrPlan fr; };
+struct F16Plan { int a_mode, bn, bk, bw, bh, bb; int pair; bool featrows; FrPlan fr; };
 static const int kF16TuneBN[3] = {64, 128, 256};
 // tune index -> (addressing mode, feature tile): 1 + mode * 3 + {64, 128, 256}; 0 = automatic
-// 1 + 3 * mode + feature tile; modes flat / im2col / tiled / patch; 13..32: the feature-row form (conv_featrows.cu)
+// 1 + 3 * mode + feature tile; modes flat / im2col / tiled / patch; 13..32: the feature-row form (conv_featrows.cu); 33..38: CTA pairs,
+// 33 + 2 * mode + {128, 256}
 constexpr int kF16TuneFeatRows = 13;
-static int f16_tune_count(const void*) { return kF16TuneFeatRows + kFrVariants; }
+constexpr int kF16TunePair = kF16TuneFeatRows + kFrVariants;
+static int f16_tune_count(const void*) { return kF16TunePair + 6; }
 constexpr size_t kF16PatchWeightBytes = 80 * 1024;                  // largest weight tensor the patch mode keeps resident
 
 static bool f16_dense(const cldnn_b200_tensor& t) { return t.py == t.px * t.x && t.pb == t.py * t.y; }
@@ -489,6 +528,11 @@ static void f16_choose_patch(int Q, int Pn, int kh, int kw, int& tw, int& th)
         }
 }
 
+static bool f16_pair_fits(const cldnn_b200_conv_params& p, int bn)
+{
+    return !p.fused_eltw && bn >= 128 && p.ofm % bn == 0 && (int64_t)p.out.b * p.out.y * p.out.x >= 2 * f16tc::kBM;
+}
+
 static bool f16_patch_fits(const cldnn_b200_conv_params& p, int bn, const char** why)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
@@ -501,7 +545,7 @@ static bool f16_patch_fits(const cldnn_b200_conv_params& p, int bn, const char**
 
 // The feature tile of an untuned launch by the estimates of conv_tile_cost.hpp; the feature-row form's variant where that is
 // cheaper, else -1.
-static void f16_choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int& bn, int& fr_variant)
+static void f16_choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, int& bn, int& pair, int& fr_variant)
 {
     const int64_t pixels = (int64_t)p.out.b * p.out.y * p.out.x, steps = (int64_t)p.kh * p.kw * (reduction_features(p) * 2 / bk);
     int64_t m_tiles = (pixels + f16tc::kBM - 1) / f16tc::kBM;
@@ -512,8 +556,13 @@ static void f16_choose_shape(const cldnn_b200_conv_params& p, int mode, int bk, 
     double best = 0.0; bn = 0; fr_variant = -1;
     for (int b : {64, 128, 256}) {
         if (p.groups > 1 ? b != 128 : (b > 64 && b / 2 >= p.ofm)) continue;      // (a grouped tile lies inside its group)
-        const double t = tile_cost(kTileCostF16, m_tiles, p.ofm, b, steps, bk, TILE_TWO_GROUPS, p.fused_eltw != 0);
-        if (bn == 0 || t < best) { best = t; bn = b; }
+        for (TileKind k : {TILE_TWO_GROUPS, TILE_PAIR}) {
+            // pairs of 256-feature tiles only: 256 -> 256 3x3 at 56x56, 32 images, 96.6 -> 90.1 us, but 384 -> 384 at 13x13, 256 images, in pairs
+            // of 128-feature tiles 124 against 102 in single tiles of 256
+            if (k == TILE_PAIR && (b != 256 || !f16_pair_fits(p, b))) continue;
+            const double t = tile_cost(kTileCostF16, m_tiles, p.ofm, b, steps, bk, k, p.fused_eltw != 0);
+            if (bn == 0 || t < best) { best = t; bn = b; pair = k == TILE_PAIR; }
+        }
     }
     int v; const double fr = fr_cost(p, v);
     if (v >= 0 && fr < best) fr_variant = v;
@@ -552,13 +601,17 @@ static bool f16_plan(const cldnn_b200_conv_params& p_in, F16Plan& pl, std::strin
     const bool im2col_ok = p.pad_x <= 127 && p.pad_y <= 127 && (p.kw - 1) * p.dil_x <= 255 && (p.kh - 1) * p.dil_y <= 255 &&
                            p.stride_x <= 8 && p.stride_y <= 8 && (int64_t)p.in.b * p.in.pb * 2 >= 131072;
     int mode = -1, bn = 0;
-    pl.featrows = false;
+    pl.featrows = false; pl.pair = 0;
     if (p.tune == 0 && !fixed) {
         const int v = fr_inner_product_variant(p);
         if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
     }
-    if (p.tune >= kF16TuneFeatRows) { pl.featrows = true; return fr_plan(p, p.tune - kF16TuneFeatRows, pl.fr, why); }
-    if (p.tune > 0) { mode = (p.tune - 1) / 3; bn = kF16TuneBN[(p.tune - 1) % 3]; }
+    if (p.tune >= kF16TunePair) {
+        if (p.tune >= kF16TunePair + 6) return no("unknown tuning index");
+        pl.pair = 1; mode = (p.tune - kF16TunePair) / 2; bn = (p.tune - kF16TunePair) % 2 ? 256 : 128;
+    }
+    else if (p.tune >= kF16TuneFeatRows) { pl.featrows = true; return fr_plan(p, p.tune - kF16TuneFeatRows, pl.fr, why); }
+    else if (p.tune > 0) { mode = (p.tune - 1) / 3; bn = kF16TuneBN[(p.tune - 1) % 3]; }
     if (mode < 0) {
         mode = is_1x1_s1 ? f16tc::A_FLAT : (im2col_ok ? f16tc::A_IM2COL : f16tc::A_TILED);
         // resident weights wherever they fit: 64 -> 64 features 3x3 at 224x224, 1 / 32 images, 14.2 against 9.5 us and 264 against 125
@@ -566,7 +619,7 @@ static bool f16_plan(const cldnn_b200_conv_params& p_in, F16Plan& pl, std::strin
         if (fixed) ;
         else if (f16_patch_fits(p, pbn, nullptr)) { mode = f16tc::A_PATCH; bn = pbn; }
         else if (mode != f16tc::A_TILED || tiled_ok) {
-            int v; f16_choose_shape(p, mode, pl.bk, bn, v);
+            int v; f16_choose_shape(p, mode, pl.bk, bn, pl.pair, v);
             if (v >= 0 && fr_plan(p, v, pl.fr, nullptr)) { pl.featrows = true; return true; }
         }
     }
@@ -577,6 +630,7 @@ static bool f16_plan(const cldnn_b200_conv_params& p_in, F16Plan& pl, std::strin
     if (p.groups > 1 && p.ofm / p.groups % bn) return no("grouped convolution: a feature tile must lie inside one group");
     if (bn == 0) bn = p.ofm > 128 ? 256 : (p.ofm > 64 ? 128 : 64);
     if (mode == f16tc::A_PATCH) { const char* m = nullptr; if (!f16_patch_fits(p, bn, &m)) return no(m); }
+    if (pl.pair && !f16_pair_fits(p, bn)) return no("CTA pairs need whole feature tiles of 128 or 256, two pixel tiles and no residual");
     pl.a_mode = mode; pl.bn = bn; pl.bw = pl.bh = pl.bb = 1;
     if (mode == f16tc::A_TILED) f16_choose_box(p.out.x, p.out.y, p.out.b, pl.bw, pl.bh, pl.bb);
     if (mode == f16tc::A_PATCH) f16_choose_patch(p.out.x, p.out.y, p.kh, p.kw, pl.bw, pl.bh);
@@ -607,15 +661,34 @@ static CUresult f16_pixel_map(CUtensorMap* tm, const F16Plan& pl, void* ptr, con
                           CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
+// programmatic stream serialisation; in pairs, clusters of two CTAs (the grid is even)
+static cudaError_t f16_launch_kernel(const void* fn, const Params& P, int grid, size_t smem, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3((unsigned)f16tc::kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = P.pair ? 2 : 1;
+    void* args[1] = {const_cast<Params*>(&P)};
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 template <int BN, bool kFused>
 static cudaError_t f16_launch_inst(const Params& P, int grid, size_t smem, cudaStream_t s)
 {
-    f16tc::conv_f16_tc_kernel<BN, kFused><<<grid, f16tc::kThreads, smem, s>>>(P);
-    return cudaGetLastError();
+    return f16_launch_kernel((const void*)f16tc::conv_f16_tc_kernel<BN, kFused>, P, grid, smem, s);
+}
+static const void* f16_kernel_pair(const Params& P)
+{
+    return P.bn == 128 ? (const void*)f16tc::conv_f16_tc_kernel<128, false, true> : (const void*)f16tc::conv_f16_tc_kernel<256, false, true>;
 }
 static cudaError_t f16_launch(const Params& P, int grid, size_t smem, cudaStream_t s)
 {
     const bool f = P.fused != 0;
+    if (P.pair) return f16_launch_kernel(f16_kernel_pair(P), P, grid, smem, s);
     switch (P.bn) {
     case 64:  return f ? f16_launch_inst<64, true>(P, grid, smem, s) : f16_launch_inst<64, false>(P, grid, smem, s);
     case 128: return f ? f16_launch_inst<128, true>(P, grid, smem, s) : f16_launch_inst<128, false>(P, grid, smem, s);
@@ -629,6 +702,7 @@ static cudaError_t f16_configure(const Params& P, int max_smem)
 {
     const bool f = P.fused != 0;
     const void* fn;
+    if (P.pair) return cudaFuncSetAttribute(f16_kernel_pair(P), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
     switch (P.bn) {
     case 64:  fn = f ? (const void*)f16tc::conv_f16_tc_kernel<64, true> : (const void*)f16tc::conv_f16_tc_kernel<64, false>; break;
     case 128: fn = f ? (const void*)f16tc::conv_f16_tc_kernel<128, true> : (const void*)f16tc::conv_f16_tc_kernel<128, false>; break;
@@ -671,10 +745,15 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
         P.tiles_w = (P.Q + pl.bw - 1) / pl.bw; P.tiles_h = (P.P + pl.bh - 1) / pl.bh;
         P.m_tiles = P.tiles_w * P.tiles_h * ((P.N + pl.bb - 1) / pl.bb);
     } else { P.tiles_w = P.tiles_h = 1; P.m_tiles = (int)((P.M_total + f16tc::kBM - 1) / f16tc::kBM); }
+    // CTA pairs take pixel tiles two at a time: an odd count gets one phantom tile past the tensor (its loads read the out-of-range
+    // fill, its stores are clipped away)
+    P.pair = pl.pair;
+    if (pl.pair) P.m_tiles = (P.m_tiles + 1) & ~1;
+    const int b_rows = pl.pair ? pl.bn / 2 : pl.bn;
     P.total_tiles = P.m_tiles * P.n_tiles;
     P.stage_rows = boxed ? pl.bw * pl.bh * pl.bb : f16tc::kBM;
-    P.a_stage_bytes = f16tc::kBM * pl.bk; P.b_stage_bytes = pl.bn * pl.bk;
-    P.a_tx_bytes = P.stage_rows * pl.bk; P.b_tx_bytes = pl.bn * pl.bk;
+    P.a_stage_bytes = f16tc::kBM * pl.bk; P.b_stage_bytes = b_rows * pl.bk;
+    P.a_tx_bytes = P.stage_rows * pl.bk; P.b_tx_bytes = b_rows * pl.bk;
     if (patch) {
         // a stage holds the kw patches of one channel chunk; the tensor core reads 128 rows from row r * bw, r < kh
         const int patch_rows = (pl.bh + p.kh - 1) * pl.bw, read_rows = (p.kh - 1) * pl.bw + f16tc::kBM;
@@ -687,7 +766,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     P.sbo = 8u * (uint32_t)pl.bk;
     P.layout_type = pl.bk == 128 ? 2u : (pl.bk == 64 ? 4u : 6u);
     // instruction descriptor: f32 accumulate, f16 x f16, both K-major, N, M
-    P.idesc = (1u << 4) | ((uint32_t)(pl.bn >> 3) << 17) | ((uint32_t)(f16tc::kBM >> 4) << 24);
+    P.idesc = (1u << 4) | ((uint32_t)(pl.bn >> 3) << 17) | ((uint32_t)((pl.pair ? 2 * f16tc::kBM : f16tc::kBM) >> 4) << 24);
     const int nbuf = pl.bn >= 256 ? 2 : 4;
     P.tmem_cols = (uint32_t)(nbuf * pl.bn);
     if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / pl.bn; P.group_ch = p.ifm; }
@@ -750,7 +829,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     {
         cuuint64_t dims[3] = {(cuuint64_t)cs, (cuuint64_t)(p.kh * p.kw), (cuuint64_t)p.ofm};
         cuuint64_t strides[2] = {(cuuint64_t)(p.w_px * 2), (cuuint64_t)(p.w_po * 2)};
-        cuuint32_t box[3] = {(cuuint32_t)bke, 1, (cuuint32_t)pl.bn};
+        cuuint32_t box[3] = {(cuuint32_t)bke, 1, (cuuint32_t)b_rows};
         cuuint32_t es[3] = {1, 1, 1};
         void* w_ptr = (char*)const_cast<void*>(a->weights) + p.w_offset * 2;
         cr = h_encode_tiled(&P.tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, w_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
@@ -767,6 +846,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
 
     int grid = ctx->prop.multiProcessorCount;
     if (grid > P.total_tiles) grid = P.total_tiles;
+    if (pl.pair) grid &= ~1;                                           // whole clusters of two (total_tiles is even)
     if (grid < 1) return fail(CLDNN_B200_INVALID_ARG, "conv_f16_tc: empty output");
     const size_t smem = smem_bytes;
     B200_CUDA(f16_configure(P, (int)max_smem));

@@ -25,7 +25,7 @@ struct TileCost {
     double overlap;                          // main loop beside the epilogue of the tile before
 };
 constexpr TileCost kTileCostI8 = {3.37, 1.05, 0.218, 0.00016, 0.868, 1.31, 0.0082, 1.23, 0.33, 0.0065, 0.0048, 1.33};
-constexpr TileCost kTileCostF16 = {3.19, 0.0, 0.240, 0.00024, 1.0, 1.09, 0.0100, 1.10, 0.40, 0.0078, 0.0078, 1.13};
+constexpr TileCost kTileCostF16 = {3.19, 0.5, 0.240, 0.00024, 0.9, 1.09, 0.0100, 1.10, 0.40, 0.0078, 0.0078, 1.13};
 
 // `m_tiles` tiles of 128 pixels, `steps` reduction steps of `bk` bytes
 inline double tile_cost(const TileCost& c, int64_t m_tiles, int64_t ofm, int bn, int64_t steps, int bk, TileKind kind, bool fused)
