@@ -342,7 +342,7 @@ constexpr int kCols[kFrCols] = {16, 32, 64, 128, 256};
 
 }  // namespace
 
-bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::string* why)
+bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::string* why, bool box)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
     if (variant < 0 || variant >= kFrVariants) return no("unknown tuning index");
@@ -363,7 +363,7 @@ bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::stri
     else if (tiled_ok) pl.mode = FR_TILED;
     else return no("neither im2col nor tiled addressing fits");
     pl.bw = pl.bh = pl.bb = 1;
-    if (pl.mode == FR_TILED) fr_choose_box(p.out.x, p.out.y, p.out.b, pl.cols, pl.bw, pl.bh, pl.bb);
+    if (pl.mode == FR_TILED && box) fr_choose_box(p.out.x, p.out.y, p.out.b, pl.cols, pl.bw, pl.bh, pl.bb);
     return true;
 }
 
@@ -410,7 +410,7 @@ double fr_cost(const cldnn_b200_conv_params& p, int& variant)
         FrPlan pl;
         const int64_t cols = kCols[v / kFrSplits], split = 1 << (v % kFrSplits), ctas = m_tiles * ((pixels + cols - 1) / cols) * split;
         const int64_t resident = (split == 8 ? 128 : (split == 4 ? 144 : 148)) * (cols == 256 ? 1 : 2);
-        if (ctas > resident || !fr_plan(p, v, pl, nullptr)) continue;
+        if (ctas > resident || !fr_plan(p, v, pl, nullptr, false)) continue;
         const double valid = (double)std::min(cols, pixels);
         const double main = (double)((steps + split - 1) / split) * (c.step + c.step_row * (double)(kRows + cols) * ((double)bk / 128.0));
         const double epi = c.col * (double)cols + c.gather * valid / (double)split + (split > 1 ? c.exchange_col * valid + c.exchange : 0.0);

@@ -34,7 +34,8 @@ constexpr int kFrSplits = 4;                 // 1, 2, 4, 8 CTAs per tile
 constexpr int kFrVariants = kFrCols * kFrSplits;
 
 // variant 0 .. kFrVariants - 1 = columns index * 4 + split index.  `p` has passed the layout checks of the calling kernel's plan.
-bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::string* why);
+// `box`: also choose the tiled mode's box (a search over the map; whether the variant fits does not depend on it).
+bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::string* why, bool box = true);
 // The variant an untuned inner product (a pointwise convolution of 1x1 maps) takes; -1: the pixel-row kernels are the better choice.
 int fr_inner_product_variant(const cldnn_b200_conv_params& p);
 // The variant with the lowest expected time (us, returned) for a convolution of any shape, among those whose CTAs are
