@@ -47,3 +47,23 @@ def test_refuses_what_it_does_not_compute(eng):
     q.out, _ = abi.tensor(abi.F16, 1, 96, 27, 27, "byxf")     # the last row of windows reaches past the map
     q.mode, q.size_x, q.size_y, q.stride_x, q.stride_y, p.lrn_size = abi.POOL_MAX, 3, 3, 2, 2, 5
     assert not eng.kernel("lrn_pool_f16_byxf").supports(p)
+
+
+@pytest.mark.parametrize("features", [16, 96])
+def test_network_on_a_planar_map(features):
+    """In a layout the joint kernel does not take (the input's own, planar) the two kernels run; either way the network's result is that of the
+    unoptimised build, up to the rounding of the device's power function."""
+    from cldnn_b200 import cldnn as cl
+    eng, dt = cl.engine(0), cl.data_types
+    lay = cl.layout(dt.f16, cl.format.bfyx, cl.tensor(3, features, 13, 11))
+    x = (np.random.default_rng(32).standard_normal((3, features, 11, 13)) * 4).astype(np.float16)
+    got = []
+    for optimize in (False, True):
+        net = cl.network(eng, cl.topology(cl.input_layout("input", lay), cl.lrn("norm", "input"), cl.pooling("pool", "norm", cl.pooling_mode.max, size=(3, 3), stride=(2, 2))),
+                         cl.build_options(optimize_data=optimize, outputs=["pool"]))
+        net.set_input_data("input", cl.memory.from_numpy(eng, x))
+        net.execute()
+        got.append(net.get_output("pool").to_numpy().astype(np.float32))
+        net.execute()
+        assert np.array_equal(net.get_output("pool").to_numpy().astype(np.float32), got[-1])
+    assert got[0].shape == got[1].shape and np.abs(got[0] - got[1]).max() <= 2e-3 * np.abs(got[0]).max()
