@@ -202,7 +202,8 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
     else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = aux->tmem_base;
-    const bool patch = P.a_mode == A_PATCH;
+    // (a pair has no patch mode; known at compile time, because a kernel's tcgen05 instructions all name the same cta_group)
+    const bool patch = !kPair && P.a_mode == A_PATCH;
     const bool boxed = P.a_mode == A_TILED || patch;
     // Each role waits for the previous kernel of the stream before it first touches memory that kernel wrote or read; weights are
     // constants of the network, and the patch mode's resident copy of them starts before that.
@@ -329,11 +330,8 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
             }
             if (kPair) {
                 // drain: the instructions read the peer's shared memory, so every one of them retires before the pair leaves
-                if (leader) tc_commit(smem_u32(&aux->drain));
-                const uint64_t t0 = globaltimer();
-                while (!mbar_try_wait(smem_u32(&aux->drain), 0u)) {
-                    if (globaltimer() - t0 > kWaitLimitNs) { atomicCAS(P.status, 0u, kErr + 8u); break; }
-                }
+                if (leader) tc_commit_pair(smem_u32(&aux->drain));
+                drain_wait(smem_u32(&aux->drain), P.status, kErr + 8u);
             }
         }
     } else if (warp == 2) {
@@ -453,8 +451,11 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
         }
     }
     tc_fence_before();
-    if (kPair) cluster_sync_all();
-    else __syncthreads();
+    __syncthreads();
+    if (kPair) {
+        if (warp == 1 && rank != 0u) drain_wait(smem_u32(&aux->drain), P.status, kErr + 9u);   // the commit's arrival has landed here too
+        cluster_sync_all();
+    }
     if (warp == 1) { tc_fence_after(); if (kPair) tmem_dealloc_pair(tmem_base, P.tmem_cols); else tmem_dealloc(tmem_base, P.tmem_cols); }
 }
 

@@ -319,7 +319,7 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
-        const bool patch = P.a_mode == A_PATCH;
+        const bool patch = !kPair && P.a_mode == A_PATCH;
         // The whole warp walks the tiles and waits on the barriers; one elected lane issues the copies.  With the loop
         // warp-uniform the compiler keeps the loop state and the copies' operands on the uniform datapath, which a loop
         // inside a one-lane branch cannot use: the role's instruction count per stage is what bounds small-tile layers.
@@ -409,7 +409,8 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
             const uint32_t full0 = smem_u32(&aux->full[0]), empty0 = smem_u32(&aux->empty[0]);
             const int kk = P.bk >> 5, stages = P.stages, k_steps = P.k_steps;
             const uint32_t idesc = P.idesc;
-            const bool patch = P.a_mode == A_PATCH;
+            // (a pair has no patch mode; known at compile time, because a kernel's tcgen05 instructions all name the same cta_group)
+            const bool patch = !kPair && P.a_mode == A_PATCH;
             const uint32_t row_step = (uint32_t)(P.bw * P.bk) >> 4;                    // patch mode: one filter row further down the patch
             const uint32_t b_row_step = (uint32_t)(P.kw * P.chunks) * b_step;          //             the weights of the next filter row
             const int kh = P.kh, kw_ = P.kw;
@@ -464,11 +465,8 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
                 if (ok && leader) { if (kPair) tc_commit_pair(smem_u32(&aux->tmem_full[acc])); else tc_commit(smem_u32(&aux->tmem_full[acc])); }
             }
             // drain: every issued MMA must have retired before TMEM is released
-            if (leader) tc_commit(smem_u32(&aux->drain));
-            const uint64_t t0 = globaltimer();
-            while (!mbar_try_wait(smem_u32(&aux->drain), 0u)) {
-                if (globaltimer() - t0 > kWaitLimitNs) { atomicCAS(P.status, 0u, kErrDrain); break; }
-            }
+            if (leader) { if (kPair) tc_commit_pair(smem_u32(&aux->drain)); else tc_commit(smem_u32(&aux->drain)); }
+            drain_wait(smem_u32(&aux->drain), P.status, kErrDrain);
         }
     } else if (warp == 2) {
         // ------------------------------ TMA store issuer --------------------------
@@ -624,8 +622,11 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
 
     tc_fence_before();
     // a pair leaves together: rank 0's tensor-core instructions read the peer's shared memory and the peer arrives on rank 0's barriers
-    if (kPair) cluster_sync_all();
-    else __syncthreads();
+    __syncthreads();
+    if (kPair) {
+        if (warp == 1 && rank != 0u) drain_wait(smem_u32(&aux->drain), P.status, kErrDrain + 1u);   // the commit's arrival has landed here too
+        cluster_sync_all();
+    }
     if (warp == 1) { tc_fence_after(); if (kPair) tmem_dealloc_pair(tmem_base, P.tmem_cols); else tmem_dealloc(tmem_base, P.tmem_cols); }
 }
 

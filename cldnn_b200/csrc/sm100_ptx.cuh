@@ -86,6 +86,15 @@ __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, vo
     return mbar_wait_slow(bar, parity, s_abort, g_status, code);
 }
 
+// The last commit of a CTA or a pair: everything it issued has retired.  Bounded, and on its own: it also follows an abort.
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t* g_status, uint32_t code)
+{
+    const uint64_t t0 = globaltimer();
+    while (!mbar_try_wait(bar, 0u)) {
+        if (globaltimer() - t0 > kWaitLimitNs) { atomicCAS(g_status, 0u, code); break; }
+    }
+}
+
 // ---- programmatic dependent launch ------------------------------------------------
 // Lets the next kernel of the stream, if it was launched with programmatic stream serialisation (the tensor-core convolutions), set up
 // and fetch its weights while this one runs; it waits for this one's end before it touches activations.  Executed once a

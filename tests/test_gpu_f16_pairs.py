@@ -55,3 +55,26 @@ def test_refusals(eng):
         for tune in list(PAIRS) + [39]:
             case.p.tune = tune
             assert not k.supports(case.p)
+
+
+def test_many_launches_in_a_row(eng):
+    """Pairs that follow one another at once, each set up while the one before still runs: its tensor memory, barriers and last commits must be
+    through before the pair leaves."""
+    case = cases.make_conv_case(63, **GEOMS["odd_tiles"][0], **F16)
+    from cldnn_b200 import engine
+    n, es = case.out_elems, 2
+    want = cases.run_oracle(case).astype(np.float32)
+    src, w, bias, outs = eng.upload(case.inp), eng.upload(case.w), eng.upload(case.bias), [eng.alloc(n * es) for _ in range(6)]
+    runs = []
+    for i, out in enumerate(outs):
+        p = cases.copy_params(case.p)
+        p.tune = 33 + 2 + i % 4                                # im2col and tiled, 128 and 256 features
+        runs.append(eng.kernel("conv_f16_tc").prepare(p, engine.make_args(input0=src, output=out, weights=w, bias=bias)))
+    for _ in range(30):
+        for r in runs:
+            r.run()
+    eng.sync()
+    assert eng.device_status() == 0
+    for out in outs:
+        got = out.read(np.float16, n).astype(np.float32)
+        assert np.abs(got - want[:n]).max() <= F16_TOL * np.abs(want[:n]).max()
