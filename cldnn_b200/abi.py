@@ -73,7 +73,7 @@ class ConvParams(C.Structure):
                 ("eltw_calibration", C.c_int32),
                 ("eltw_stride_x", C.c_int32), ("eltw_stride_y", C.c_int32),
                 ("in_out_opt", C.c_int32),
-                ("tune", C.c_int32), ("epilogue_order", C.c_int32), ("reserved", C.c_int32 * 6)]
+                ("tune", C.c_int32), ("epilogue_order", C.c_int32), ("constant_params", C.c_int32), ("reserved", C.c_int32 * 5)]
 
 
 class Args(C.Structure):

@@ -63,6 +63,7 @@ struct alignas(64) Params {
     int32_t b_total_bytes, patch_alloc;      // patch mode: all taps' weights (resident), bytes reserved per patch
     int32_t batch_tiles;                     // batched GEMM view: tiles per batch, the weight 'tap' is the batch index (0 = plain convolution)
     int32_t ofm, fused, bias_dtype, act, eltw_act;
+    int32_t early_params;                    // weights may be read before the previous kernel has ended
     int32_t pair;                            // CTA pairs: m_tiles is even, the weight box holds bn / 2 rows
     int32_t group_tiles, group_ch;           // grouped: feature tiles per group (0: one group), its input features
     float act_m, act_n, eltw_m, eltw_n;
@@ -205,8 +206,8 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
     // (a pair has no patch mode; known at compile time, because a kernel's tcgen05 instructions all name the same cta_group)
     const bool patch = !kPair && P.a_mode == A_PATCH;
     const bool boxed = P.a_mode == A_TILED || patch;
-    // Each role waits for the previous kernel of the stream before it first touches memory that kernel wrote or read; weights are
-    // constants of the network, and the patch mode's resident copy of them starts before that.
+    // Each role waits for the previous kernel of the stream before it first touches memory that kernel wrote or read; the patch mode's
+    // resident copy of the weights starts before that where they are constants of the network.
     griddep_launch_dependents();
 
     if (warp == 0) {
@@ -217,6 +218,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
             const bool leader = elect_one();
             int stage = 0; uint32_t phase = 0; int64_t issued = 0; bool ok = true;
             const int bke = P.bk >> 1;                               // channels per chunk
+            if (!P.early_params) griddep_wait();
             if (patch && leader && blockIdx.x < (unsigned)P.total_tiles) {
                 // every tap's weights, once per CTA (one feature tile in this mode)
                 const uint32_t bf = smem_u32(&aux->b_full);
@@ -749,6 +751,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     // CTA pairs take pixel tiles two at a time: an odd count gets one phantom tile past the tensor (its loads read the out-of-range
     // fill, its stores are clipped away)
     P.pair = pl.pair;
+    P.early_params = p.constant_params;
     if (pl.pair) P.m_tiles = (P.m_tiles + 1) & ~1;
     const int b_rows = pl.pair ? pl.bn / 2 : pl.bn;
     P.total_tiles = P.m_tiles * P.n_tiles;

@@ -10,8 +10,9 @@
 //   reading the others' partial sums through distributed shared memory (no workspace in HBM, no atomics; a fixed order of the
 //   fp32 sums).  Four consecutive features of one pixel per thread: a warp stores 128 features of a pixel contiguously.
 //   Warp 0 loads, warp 1 issues the tensor-core instructions, all eight warps run the epilogue.
-// Launched with programmatic stream serialisation: the weights of the first stages are constants of the network and are
-// requested before the previous kernel has finished; activations only after griddepcontrol.wait.
+// Launched with programmatic stream serialisation: where the parameters are constants of the network (early_params) the weights of the
+// first stages are requested and the epilogue's constants read before the previous kernel has finished; activations only after
+// griddepcontrol.wait.
 #include <cuda.h>
 #include <algorithm>
 #include <mutex>
@@ -39,6 +40,7 @@ struct alignas(64) FrParams {
     int32_t stages, a_stage_bytes, b_stage_bytes, tx_bytes, ring_bytes;
     uint32_t sbo, layout_type, idesc, tmem_cols;
     int32_t ofm;
+    int32_t early_params;                     // weights and per-feature constants may be read before the previous kernel has ended
     int32_t group_tiles, group_ch;            // grouped: feature tiles per group (0: one group), its input features
     int64_t out_px, out_py, out_pb, out_off, el_px, el_py, el_pb, el_off;
     int32_t el_sx, el_sy;
@@ -136,7 +138,8 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
     const uint32_t tmem_base = aux->tmem_base;
     griddep_launch_dependents();
 
-    // constants of the epilogue (of the network too): fetched under the previous kernel's tail and the main loop
+    // constants of the epilogue: fetched under the previous kernel's tail, unless that kernel may be computing them, and the main loop
+    if (!P.early_params) griddep_wait();
     const EpiCfg& c = P.epi;
     const int f = m_tile * kRows + lane * 4;                         // this thread's four features
     const int nf = min(4, P.ofm - f);
@@ -452,7 +455,7 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     P.idesc = f16 ? (1u << 4) : ((2u << 4) | (1u << 7) | ((p.in.dtype == CLDNN_B200_U8 ? 0u : 1u) << 10));
     P.idesc |= ((uint32_t)(P.cols >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
     P.tmem_cols = (uint32_t)(P.cols < 32 ? 32 : P.cols);
-    P.ofm = p.ofm;
+    P.ofm = p.ofm; P.early_params = p.constant_params;
     if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / kRows; P.group_ch = p.ifm; }
     const cldnn_b200_tensor& et = p.in_out_opt ? p.out : p.eltw;
     P.out_px = p.out.px; P.out_py = p.out.py; P.out_pb = p.out.pb; P.out_off = p.out.offset;

@@ -670,6 +670,7 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
         P.m_tiles = (int)((P.M_total + kBM - 1) / kBM);
     }
     P.pair = pl.pair;
+    P.early_params = p.constant_params;
     // CTA pairs take pixel tiles two at a time: an odd count gets one phantom tile past the tensor (its loads read the
     // out-of-range fill, its stores are clipped away); each CTA loads half of the feature tile's weight rows
     if (pl.pair) P.m_tiles = (P.m_tiles + 1) & ~1;

@@ -314,8 +314,9 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
     const uint32_t tmem_base = aux->tmem_base;
     griddep_launch_dependents();
     // Each role waits for the previous kernel of the stream itself, right before it first touches memory that kernel wrote or
-    // read (activations, residual, output).  The weights are constants of the network: the producer starts their resident
-    // copy before it waits, so that copy runs under the previous kernel's tail.  The MMA issuers touch no global memory.
+    // read (activations, residual, output).  Where weights and per-feature constants are the network's (early_params), the producer starts
+    // the resident copy of the weights before it waits and the epilogue fetches the constants, so that both run under the previous
+    // kernel's tail; otherwise that kernel may be computing them.  The MMA issuers touch no global memory.
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
@@ -329,6 +330,7 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
             // output features would otherwise fetch the same few KB again for every tile -- as many requests as the
             // activation tile itself costs, for nothing.
             const bool resb = patch || P.b_resident != 0;
+            if (!P.early_params) griddep_wait();
             if (leader && resb && blockIdx.x < (unsigned)P.total_tiles) {
                 // every filter tap (and channel chunk) of every feature tile, once per CTA
                 const uint32_t bf = smem_u32(&aux->b_full);
@@ -546,6 +548,7 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
         const bool with_oqf = (P.fast_variant & 8) != 0;            // uniform O_QF after the dequantisation
         const float oqf = c.o_qf, oqf_abs = with_oqf ? fabsf(c.o_qf) : 1.0f;
         int cur_n_tile = -1; bool ok = true; bool wide = false;
+        if (!P.early_params) griddep_wait();
         int t = group;
         TileWalk walk; walk.init(P, blockIdx.x + group * gridDim.x, kGroups * gridDim.x);
         walk.mode = A_FLAT;                                         // only the feature tile is needed here
@@ -571,7 +574,7 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
                 if (lane == 0) aux->wide[group][quad] = w ? 1u : 0u;
                 named_bar_sync(1 + group, 128);
                 wide = (aux->wide[group][0] | aux->wide[group][1] | aux->wide[group][2] | aux->wide[group][3]) != 0u;
-                if (cur_n_tile < 0) griddep_wait();                 // (the constants above are the network's: fetched before the wait)
+                if (cur_n_tile < 0) griddep_wait();
                 cur_n_tile = n_tile;
             }
             if (!mbar_wait(smem_u32(&aux->tmem_full[acc]), par, s_abort, P.status, kErrEpilogue)) { ok = false; break; }

@@ -1016,6 +1016,12 @@ void network_impl::prepare_kernel(node* n)
             cldnn_b200_args ta = a; ta.weights = n->packed_weights.device_ptr();
             if (taken) {
                 a = ta; cp = tp;
+                // The kernel may read its parameters ahead of the previous kernel's end when nothing in flight can be writing them: they are
+                // data, the weights were packed above, and a captured pass begins only when everything before it has ended (launched one
+                // by one, a pass follows its predecessor's kernels, whose results may be this network's data, as closely as its own).
+                bool constant = opts.use_graph && !eng->profiling;
+                for (node* d : {n->bias, n->wq, n->oc, n->ec}) constant = constant && (!d || d->constant());
+                cp.constant_params = constant ? 1 : 0;
                 // Winograd F(2x2, 3x3) beside the direct form, behind a gate modelled on should_use_winograd_2x3_s1
                 // (src/layout_optimizer.cpp:34-53): 3x3 stride-1 undilated ungrouped fp16 convolutions whose feature counts are
                 // multiples of 64, maps of at least 8x8, an input that is neither tiny nor so large that the transformed
@@ -1036,7 +1042,7 @@ void network_impl::prepare_kernel(node* n)
                     cands.push_back("conv_f16_winograd");
                 }
                 // the tile shape does not depend on whether the residual is read from the output buffer: one cache entry for both
-                cldnn_b200_conv_params key = cp; key.in_out_opt = 0; key.tune = 0;
+                cldnn_b200_conv_params key = cp; key.in_out_opt = 0; key.tune = 0; key.constant_params = 0;
                 finish(cands, &cp, sizeof(cp), [&](int tn) { cp.tune = tn; }, cands.size() > 1, &key);
                 if (n->kernel != "conv_f16_winograd" && n->scratch) {      // the direct form won: the workspace goes back
                     // (the prepared launch of the direct kernel never looks at the scratch pointer)

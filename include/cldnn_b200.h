@@ -135,7 +135,10 @@ typedef struct cldnn_b200_conv_params {
     /* implementation choice (tuning index of the selected kernel)          */
     int32_t tune;
     int32_t epilogue_order;      /* CLDNN_B200_EPILOGUE_*: whose operation order the quantised epilogue follows */
-    int32_t reserved[6];
+    /* 1: weights, bias and factors hold their final values before the kernel ahead of this launch in the stream starts (constants of a
+     * network); kernels launched ahead of that kernel's end may then read them early.  0: they may be that kernel's output.  */
+    int32_t constant_params;
+    int32_t reserved[5];
 } cldnn_b200_conv_params;
 
 /* Arguments by role, in the order of kernel_selector's ArgumentDescriptor

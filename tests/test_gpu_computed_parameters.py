@@ -1,0 +1,80 @@
+"""Parameters that are not constants: weights, bias and factors written by the kernel in front of a convolution.  That kernel lets the convolution start
+before it has ended, so the convolution reads its parameters only after it has waited."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import cases
+from cldnn_b200 import abi
+
+pytestmark = pytest.mark.gpu
+F16_TOL = 2.0 ** -10                                   # one rounding to half of fp32 sums in another order
+
+
+@pytest.fixture(scope="module")
+def eng():
+    from cldnn_b200 import engine
+    e = engine.Engine(0)
+    yield e
+    e.close()
+
+
+def slow_copy(eng, src, dst, nbytes, taps):
+    """A prepared launch that writes `nbytes` (a multiple of 16) from src to dst as the maximum over a window of taps x taps equal pixels: one thread per 16
+    bytes, so it runs long and leaves most of the device free.  Every pixel of the window is the same memory (pitches of zero)."""
+    from cldnn_b200 import engine
+    p = abi.PoolParams()
+    p.in_, _ = abi.tensor(abi.U8, 1, nbytes, taps, taps, "byxf")
+    p.out, _ = abi.tensor(abi.U8, 1, nbytes, 1, 1, "byxf")
+    p.in_.px = p.in_.py = 0
+    p.mode, p.size_x, p.size_y, p.stride_x, p.stride_y = abi.POOL_MAX, taps, taps, 1, 1
+    return eng.kernel("pooling_i8_byxf").prepare(p, engine.make_args(input0=src, output=dst))
+
+
+I8 = dict(N=1, C=64, K=64, H=20, W=20, out_dtype=np.uint8)
+DEEP = dict(N=1, C=256, K=192, H=7, W=7, out_dtype=np.uint8)
+HALF = dict(in_dtype=np.float16, out_dtype=np.float16, quant=False, bias="f32")
+FORMS = {
+    # kernel, tuning index, case
+    "i8_patch": ("conv_i8_tc", 26, dict(I8, K=128)),
+    "i8_tiled": ("conv_i8_tc", 10, I8),
+    "i8_resident": ("conv_i8_tc", 2, dict(I8, N=40, H=33, W=31, kh=1, kw=1, pad=0)),
+    "i8_pair": ("conv_i8_tc", 49, dict(I8, K=128, N=2)),
+    "i8_rows_split": ("conv_i8_tc", 51 + 4 * 2 + 3, DEEP),
+    "i8_rows": ("conv_i8_tc", 51 + 4 * 1, DEEP),
+    "f16_patch": ("conv_f16_tc", 10, dict(N=1, C=64, K=64, H=20, W=20, **HALF)),
+    "f16_rows_split": ("conv_f16_tc", 13 + 4 * 2 + 2, dict(DEEP, **HALF)),
+    "untuned_i8": ("conv_i8_tc", 0, DEEP),
+    "untuned_f16": ("conv_f16_tc", 0, dict(DEEP, **HALF)),
+}
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+def test_written_by_the_kernel_in_front(eng, form):
+    from cldnn_b200 import engine
+    kernel, tune, geom = FORMS[form]
+    case = cases.make_conv_case(81, **geom)
+    want, n, es = cases.run_oracle(case), case.out_elems, np.dtype(geom["out_dtype"]).itemsize
+    arrays = {k: v for k, v in dict(weights=case.w, bias=case.bias, quant=case.quant).items() if v is not None}
+    src, out = eng.upload(case.inp), eng.alloc(n * es)
+    p = cases.copy_params(case.p)
+    p.tune = tune
+    assert p.constant_params == 0 and eng.kernel(kernel).supports(p)
+    for late in arrays:
+        bufs = {k: eng.upload(v) for k, v in arrays.items()}
+        final, stale = eng.upload(arrays[late]), np.ones_like(arrays[late])
+        copy = slow_copy(eng, final, bufs[late], arrays[late].nbytes, 64)
+        conv = eng.kernel(kernel).prepare(p, engine.make_args(input0=src, output=out, **bufs))
+        for _ in range(3):
+            bufs[late].write(stale)
+            copy.run()
+            conv.run()
+            eng.sync()
+            assert eng.device_status() == 0
+            got = out.read(np.dtype(geom["out_dtype"]), n)
+            if es == 1:
+                assert np.array_equal(got, want[:n]), late
+            else:
+                w32 = want[:n].astype(np.float32)
+                assert np.abs(got.astype(np.float32) - w32).max() <= F16_TOL * np.abs(w32).max(), late
