@@ -240,6 +240,8 @@ struct node {
     std::vector<node*> deps;            // data inputs
     std::vector<node*> users;
     node *weights = nullptr, *bias = nullptr, *wq = nullptr, *oc = nullptr, *ec = nullptr;
+    int param_uses = 0;                 // nodes that read this one as weights, bias or factors (they are not in `users`)
+    std::vector<node*> params() const { std::vector<node*> v; for (node* d : {weights, bias, wq, oc, ec}) if (d) v.push_back(d); return v; }
     layout out;
     bool is_output = false;
     bool removed = false;
@@ -333,12 +335,13 @@ public:
 
 void network_impl::link()
 {
-    for (auto& up : nodes) { up->deps.clear(); up->users.clear(); }
+    for (auto& up : nodes) { up->deps.clear(); up->users.clear(); up->param_uses = 0; }
     for (auto& up : nodes) {
         node* n = up.get(); if (n->removed) continue;
         for (auto& id : n->p.input) { node* d = get(id); n->deps.push_back(d); d->users.push_back(n); }
         n->weights = opt(n->p.weights); n->bias = opt(n->p.bias); n->wq = opt(n->p.weights_quantization_factors);
         n->oc = opt(n->p.output_calibration_factors); n->ec = opt(n->p.eltw_output_calibration_factors);
+        for (node* d : n->params()) ++d->param_uses;
     }
 }
 
@@ -351,7 +354,7 @@ void network_impl::sort()
         if (done.count(n) || n->removed) return;
         done.insert(n);
         for (node* d : n->deps) visit(d);
-        for (node* d : {n->weights, n->bias, n->wq, n->oc, n->ec}) if (d) visit(d);
+        for (node* d : n->params()) visit(d);
         order.push_back(n);
     };
     for (auto& up : nodes) visit(up.get());
@@ -437,7 +440,7 @@ void network_impl::fuse_activations()
         node* prod = a->deps[0];
         const std::string& t = prod->p.type;
         if (!(t == "convolution" || t == "fused_conv_eltwise" || t == "eltwise" || t == "fully_connected" || t == "pooling")) continue;
-        if (prod->users.size() != 1 || prod->is_output) continue;
+        if (prod->users.size() != 1 || prod->param_uses || prod->is_output) continue;
         const bool on_eltw = t == "fused_conv_eltwise";
         int32_t& slot = on_eltw ? prod->eltw_act : prod->act;
         const bool own = on_eltw ? prod->p.eltw_activation : prod->p.with_activation;
@@ -462,7 +465,7 @@ void network_impl::fuse_lrn_pool()
         node* n = nodes[i].get();
         if (n->removed || n->p.type != "pooling" || n->deps.size() != 1 || n->lrn_size || n->act != CLDNN_B200_ACT_NONE) continue;
         node* l = n->deps[0];
-        if (l->p.type != "lrn" || l->users.size() != 1 || l->is_output || l->deps.size() != 1 || l->deps[0]->out.data_type != data_types::f16) continue;
+        if (l->p.type != "lrn" || l->users.size() != 1 || l->param_uses || l->is_output || l->deps.size() != 1 || l->deps[0]->out.data_type != data_types::f16) continue;
         const bool window = n->p.pool_mode == pooling_mode::max && !n->p.global_pooling && n->p.size.x == 3 && n->p.size.y == 3 && n->p.stride.x == 2 &&
                             n->p.stride.y == 2 && n->p.input_offset.x == 0 && n->p.input_offset.y == 0;
         const tensor& ls = l->out.size; const tensor& os = n->out.size;
@@ -488,7 +491,7 @@ void network_impl::fuse_conv_eltwise()
         if (e->removed || e->p.type != "eltwise" || e->p.mode != eltwise_mode::sum || e->deps.size() != 2) continue;
         node* a = e->deps[0]; node* b = e->deps[1];
         auto fusable = [&](node* c) {
-            if (c->p.type != "convolution" || c->users.size() != 1 || c->is_output || c->p.groups != 1) return false;
+            if (c->p.type != "convolution" || c->users.size() != 1 || c->param_uses || c->is_output || c->p.groups != 1) return false;
             if (!opts.fuse_any_conv_eltwise) {
                 const layout& w = c->weights->out;
                 if (w.size.x != 1 || w.size.y != 1 || c->p.stride.x != 1 || c->p.stride.y != 1) return false;
@@ -613,7 +616,7 @@ void network_impl::conv_eltw_read_write_opt()
     for (node* n : order) {
         if (n->removed || n->p.type != "fused_conv_eltwise" || n->deps.size() != 2) continue;
         node* r = n->deps[1];
-        if (r == n->deps[0] || r->constant() || r->p.type == "input_layout" || r->is_output) continue;
+        if (r == n->deps[0] || r->constant() || r->p.type == "input_layout" || r->is_output || r->param_uses) continue;
         if (!(r->out == n->out) || n->p.eltw_stride.x != 1 || n->p.eltw_stride.y != 1) continue;
         bool safe = true;
         for (node* u : r->users) safe &= u == n || u->order < n->order;
@@ -1180,6 +1183,7 @@ void network_impl::allocate_and_prepare()
     std::vector<int> last_use(order.size(), -1);
     for (node* n : order) {
         for (node* d : n->deps) last_use[d->order] = std::max(last_use[d->order], n->order);
+        for (node* d : n->params()) last_use[d->order] = std::max(last_use[d->order], n->order);   // a bias may be computed by the network
         if (n->is_output) last_use[n->order] = 1 << 30;
     }
     std::multimap<size_t, std::shared_ptr<block>> free_blocks;

@@ -1,5 +1,5 @@
 """Parameters that are not constants: weights, bias and factors written by the kernel in front of a convolution.  That kernel lets the convolution start
-before it has ended, so the convolution reads its parameters only after it has waited."""
+before it has ended, so the convolution reads its parameters only after it has waited.  And a bias that a network computes for itself."""
 import ctypes as C
 
 import numpy as np
@@ -7,6 +7,7 @@ import pytest
 
 import cases
 from cldnn_b200 import abi
+from cldnn_b200 import cldnn as cl
 
 pytestmark = pytest.mark.gpu
 F16_TOL = 2.0 ** -10                                   # one rounding to half of fp32 sums in another order
@@ -78,3 +79,40 @@ def test_written_by_the_kernel_in_front(eng, form):
             else:
                 w32 = want[:n].astype(np.float32)
                 assert np.abs(got.astype(np.float32) - w32).max() <= F16_TOL * np.abs(w32).max(), late
+
+
+def _weights(rng, k, c, f):
+    return (rng.standard_normal((k, c, f, f)) / np.sqrt(c * f * f)).astype(np.float16)
+
+
+def _run(eng, prims, x, lay, outputs, **options):
+    net = cl.network(eng, cl.topology(cl.input_layout("input", lay), *prims), cl.build_options(outputs=outputs, **options))
+    net.set_input_data("input", cl.memory.from_numpy(eng, x))
+    net.execute()
+    got = []
+    for _ in range(20):
+        net.execute()
+        got = [net.get_output(o).to_numpy().astype(np.float32) for o in outputs]
+    return got
+
+
+@pytest.mark.parametrize("optimize", [False, True])
+@pytest.mark.parametrize("graph", [False, True])
+def test_bias_from_an_inner_product(optimize, graph):
+    """The bias is computed early, other small results follow it, and the convolution that reads it comes last: its buffer is nobody else's until then."""
+    eng, rng, dt = cl.engine(0), np.random.default_rng(51), cl.data_types
+    c, k = 64, 128
+    lay = cl.layout(dt.f16, cl.format.bfyx, cl.tensor(1, c, 7, 7))
+    x = rng.standard_normal((1, c, 7, 7)).astype(np.float16)
+    consts = {"w0": _weights(rng, c, c, 3), "wf": _weights(rng, k, c, 1), "wg": _weights(rng, k, c, 1), "w1": _weights(rng, k, c, 3)}
+    mems = {n: cl.memory.from_numpy(eng, a) for n, a in consts.items()}
+    datas = [cl.data(n, m) for n, m in mems.items()]
+    head = [cl.convolution("conv0", "input", "w0", input_offset=(-1, -1)), cl.pooling("mean", "conv0", cl.pooling_mode.average, global_pooling=True),
+            cl.fully_connected("bias", "mean", "wf"), cl.fully_connected("other", "mean", "wg"), cl.activation("square", "other", cl.activation_func.square)]
+    last = [cl.convolution("conv1", "input", "w1", "bias", input_offset=(-1, -1))]
+    got = _run(eng, datas + head + last, x, lay, ["conv1", "square"], optimize_data=optimize, use_graph=graph)
+    # the same with the bias read back and given as data
+    bias, = _run(eng, datas[:2] + head[:3], x, lay, ["bias"], optimize_data=optimize, use_graph=graph)
+    given = cl.memory.from_numpy(eng, bias.reshape(1, k, 1, 1).astype(np.float16))
+    want, = _run(eng, [datas[3], cl.data("bias", given)] + last, x, lay, ["conv1"], optimize_data=optimize, use_graph=graph)
+    assert np.abs(bias).max() > 0 and np.array_equal(got[0], want)
