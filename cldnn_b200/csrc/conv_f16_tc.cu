@@ -286,6 +286,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
         // (in a pair only the CTA of rank 0 issues; its instructions and commits act on both CTAs)
         if (!kPair || rank == 0u) {
             const bool leader = elect_one();
+            griddep_wait();                                            // (the bounded waits below count their own kernel's time only)
             const uint32_t hi = desc_hi(P.sbo, P.layout_type);
             const uint32_t a_lo0 = desc_lo(a_base), b_lo0 = desc_lo(b_base);
             const uint32_t a_step = (uint32_t)P.a_stage_bytes >> 4, b_step = (uint32_t)P.b_stage_bytes >> 4;

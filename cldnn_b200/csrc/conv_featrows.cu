@@ -208,6 +208,7 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
         // ------------------------------ MMA issuer --------------------------------
         const bool leader = elect_one();
         const int kk = P.bk >> 5;                                    // one instruction consumes 32 bytes of K
+        griddep_wait();                                              // (the bounded waits below count their own kernel's time only)
         for (int i = 0; i < steps; ++i) {
             const int st = i % P.stages;
             if (!__all_sync(0xffffffffu, mbar_wait_lean(smem_u32(&aux->full[st]), (uint32_t)(i / P.stages) & 1u, s_abort, P.status, kFrErr + 1u))) break;

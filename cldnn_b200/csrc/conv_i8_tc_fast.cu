@@ -316,7 +316,8 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
     // Each role waits for the previous kernel of the stream itself, right before it first touches memory that kernel wrote or
     // read (activations, residual, output).  Where weights and per-feature constants are the network's (early_params), the producer starts
     // the resident copy of the weights before it waits and the epilogue fetches the constants, so that both run under the previous
-    // kernel's tail; otherwise that kernel may be computing them.  The MMA issuers touch no global memory.
+    // kernel's tail; otherwise that kernel may be computing them.  The MMA issuers touch no global memory; they wait too, so that their
+    // bounded waits for operands do not count the previous kernel's time.
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
@@ -405,6 +406,7 @@ conv_i8_tc_fast_kernel(const __grid_constant__ TcParams P)
         // In a pair only the CTA of rank 0 issues; its instructions and commits act on both CTAs.
         if (!kPair || rank == 0u) {
             const bool leader = ptx::elect_one();
+            griddep_wait();
             const uint32_t hi = desc_hi(P.sbo, P.layout_type);
             const uint32_t a_lo0 = desc_lo(a_base), b_lo0 = desc_lo(b_base);
             const uint32_t a_step = (uint32_t)P.a_stage_bytes >> 4, b_step = (uint32_t)P.b_stage_bytes >> 4;

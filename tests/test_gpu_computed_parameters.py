@@ -81,6 +81,33 @@ def test_written_by_the_kernel_in_front(eng, form):
                 assert np.abs(got.astype(np.float32) - w32).max() <= F16_TOL * np.abs(w32).max(), late
 
 
+@pytest.mark.parametrize("form", ["i8_patch", "i8_tiled", "i8_pair", "i8_rows_split", "f16_patch", "f16_rows_split", "untuned_f16"])
+def test_behind_a_kernel_that_runs_longer_than_the_waits(eng, form):
+    """A launch set up ahead of a previous kernel that takes 2.6 s more: the limit of 2 s on waits inside a kernel is for that kernel's own time."""
+    from cldnn_b200 import engine
+    kernel, tune, geom = FORMS[form]
+    case = cases.make_conv_case(82, **geom)
+    want, n, dt = cases.run_oracle(case), case.out_elems, np.dtype(geom["out_dtype"])
+    arrays = {k: v for k, v in dict(weights=case.w, bias=case.bias, quant=case.quant).items() if v is not None}
+    src, out, bufs = eng.upload(case.inp), eng.alloc(n * dt.itemsize), {k: eng.upload(v) for k, v in arrays.items()}
+    p = cases.copy_params(case.p)
+    p.tune = tune
+    conv = eng.kernel(kernel).prepare(p, engine.make_args(input0=src, output=out, **bufs))
+    scrap = eng.alloc(256)
+    probe = slow_copy(eng, scrap, scrap, 16, 512).time_ns(1, 3)
+    slow = slow_copy(eng, scrap, scrap, 16, min(int(512 * (2.6e9 / probe) ** 0.5), 46000))   # at most 2^31 taps
+    slow.run()
+    conv.run()
+    eng.sync()
+    assert eng.device_status() == 0
+    got = out.read(dt, n)
+    if dt.itemsize == 1:
+        assert np.array_equal(got, want[:n])
+    else:
+        w32 = want[:n].astype(np.float32)
+        assert np.abs(got.astype(np.float32) - w32).max() <= F16_TOL * np.abs(w32).max()
+
+
 def _weights(rng, k, c, f):
     return (rng.standard_normal((k, c, f, f)) / np.sqrt(c * f * f)).astype(np.float16)
 
