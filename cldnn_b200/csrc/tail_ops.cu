@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cuda_fp16.h>
 #include "engine.hpp"
+#include "reorder_tile.hpp"
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -867,7 +868,7 @@ reorder_ref_kernel(const __grid_constant__ cldnn_b200_reorder_params p, const vo
 // element, whatever the planes' size keeps aligned).  13 - 18 us for the same tensor, 2.9 - 4.0 TB/s; tiles are small so that one
 // image still makes many blocks.
 // (No early release of dependents: weights are packed with this kernel, and convolutions fetch weights before they wait.)
-constexpr int kTileF = 64, kTileP = 64, kTilePitch = kTileP + 2;
+constexpr int kTilePitch = kTileP + 2;
 template <class T, int VB, bool kToByxf>
 __global__ void __launch_bounds__(256)
 reorder_tile_kernel(const T* __restrict__ in, T* __restrict__ out, int F, int Fs, int HW, int64_t plane_pf, int64_t plane_pb, int64_t inner_px, int64_t inner_pb)
@@ -901,13 +902,16 @@ reorder_tile_kernel(const T* __restrict__ in, T* __restrict__ out, int F, int Fs
     auto inner = [&](bool load) {
         for (int i = threadIdx.x; i < kTileP * (kTileF / VF); i += 256) {
             const int p = i / (kTileF / VF), f = (i - p * (kTileF / VF)) * VF;
-            if (p0 + p >= HW || f0 + f >= Fs) continue;                        // the stored feature count is in whole vectors
+            if (p0 + p >= HW || f0 + f >= (load ? F : Fs)) continue;           // (written features are in whole vectors)
             union { T e[VF]; uint4 q; } v;
             const int64_t at = b * inner_pb + (int64_t)(p0 + p) * inner_px + f0 + f;
             if (load) {
-                v.q = *reinterpret_cast<const uint4*>(in + at);
+                if (f0 + f + VF <= F) {
+                    v.q = *reinterpret_cast<const uint4*>(in + at);
 #pragma unroll
-                for (int k = 0; k < VF; ++k) tile[f + k][p] = v.e[k];
+                    for (int k = 0; k < VF; ++k) tile[f + k][p] = v.e[k];
+                } else
+                    for (int k = 0; k < F - (f0 + f); ++k) tile[f + k][p] = in[at + k];   // what lies behind the last feature need not belong to the tensor
             } else {
 #pragma unroll
                 for (int k = 0; k < VF; ++k) v.e[k] = tile[f + k][p];
@@ -921,34 +925,22 @@ reorder_tile_kernel(const T* __restrict__ in, T* __restrict__ out, int F, int Fs
 }
 
 template <class T, bool kToByxf>
-static std::function<cudaError_t(cudaStream_t)> reorder_tile_launch(int vb, dim3 grid, const void* in, void* out, int F, int Fs, int HW, int64_t ppf, int64_t ppb, int64_t ipx, int64_t ipb)
+static std::function<cudaError_t(cudaStream_t)> reorder_tile_launch(const ReorderTilePlan& t, const void* in, void* out)
 {
-    auto* k = vb == 16 ? reorder_tile_kernel<T, 16, kToByxf> : (vb == 4 ? reorder_tile_kernel<T, 4, kToByxf> : reorder_tile_kernel<T, (int)sizeof(T), kToByxf>);
-    return [=](cudaStream_t s) { return launch_dependent(k, grid, 256, s, (const T*)in, (T*)out, F, Fs, HW, ppf, ppb, ipx, ipb); };
+    auto* k = t.vector == 16 ? reorder_tile_kernel<T, 16, kToByxf> : (t.vector == 4 ? reorder_tile_kernel<T, 4, kToByxf> : reorder_tile_kernel<T, (int)sizeof(T), kToByxf>);
+    const T* src = (const T*)in + t.in_offset; T* dst = (T*)out + t.out_offset;
+    return [=](cudaStream_t s) {
+        return launch_dependent(k, dim3(t.grid_x, t.grid_y, t.grid_z), 256, s, src, dst, t.features, t.stored, t.pixels, t.plane_pf, t.plane_pb, t.inner_px, t.inner_pb);
+    };
 }
 
 // the tile kernel's launch, or an empty function when the two layouts are not its pair
 static std::function<cudaError_t(cudaStream_t)> reorder_tile_form(const cldnn_b200_reorder_params& p, const void* in, void* out)
 {
-    const int es = dtype_bytes(p.in.dtype);
-    if (p.has_mean || p.in.dtype != p.out.dtype || (es != 1 && es != 2)) return {};
-    const bool to = p.in.px == 1 && p.out.pf == 1 && p.out.px > 1, from = p.in.pf == 1 && p.in.px > 1 && p.out.px == 1;
-    if (!to && !from) return {};
-    const cldnn_b200_tensor& pl = to ? p.in : p.out; const cldnn_b200_tensor& nn = to ? p.out : p.in;
-    const int64_t HW = (int64_t)pl.y * pl.x, Fs = to ? p.out.f : (p.in.f + 15) / 16 * 16, vf = 16 / es;
-    if (HW < 8 || pl.py != pl.x || nn.py != nn.px * nn.x || HW >= (1 << 30)) return {};
-    if (nn.px % vf || nn.pb % vf || nn.offset % vf || Fs % vf || Fs > nn.px || (!to && p.out.f != p.in.f)) return {};
-    const char* ia = (const char*)in + (int64_t)p.in.offset * es; char* oa = (char*)out + (int64_t)p.out.offset * es;
-    if ((uintptr_t)(to ? oa : ia) & 15) return {};
-    int vb = es;
-    for (int v : {16, 4}) if ((HW * es) % v == 0 && (pl.pf * es) % v == 0 && (pl.pb * es) % v == 0 && ((uintptr_t)(to ? ia : oa)) % v == 0) { vb = v; break; }
-    const dim3 grid((unsigned)((Fs + kTileF - 1) / kTileF), (unsigned)((HW + kTileP - 1) / kTileP), (unsigned)p.in.b);
-    if (grid.y > 65535u || grid.z > 65535u || grid.z == 0) return {};
-    const int F = p.in.f;
-    if (es == 1) return to ? reorder_tile_launch<uint8_t, true>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb)
-                           : reorder_tile_launch<uint8_t, false>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb);
-    return to ? reorder_tile_launch<uint16_t, true>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb)
-              : reorder_tile_launch<uint16_t, false>(vb, grid, ia, oa, F, (int)Fs, (int)HW, pl.pf, pl.pb, nn.px, nn.pb);
+    ReorderTilePlan t;
+    if (!reorder_tile_plan(p, (uintptr_t)in, (uintptr_t)out, t)) return {};
+    if (t.element == 1) return t.to_inner ? reorder_tile_launch<uint8_t, true>(t, in, out) : reorder_tile_launch<uint8_t, false>(t, in, out);
+    return t.to_inner ? reorder_tile_launch<uint16_t, true>(t, in, out) : reorder_tile_launch<uint16_t, false>(t, in, out);
 }
 
 static bool reorder_supports(const void* vp) { const auto& p = *(const cldnn_b200_reorder_params*)vp; return p.in.b == p.out.b && p.in.y == p.out.y && p.in.x == p.out.x && p.out.f >= p.in.f; }

@@ -39,3 +39,28 @@ def test_planar_to_inner_and_back(eng, dtype, shape):
     back = eng.upload(np.full(n, 77, dtype=a.dtype))
     eng.kernel("reorder_ref").launch(q, engine.make_args(input0=dst, output=back))
     assert np.array_equal(back.read(a.dtype), a.reshape(-1))
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.float16])
+@pytest.mark.parametrize("f,at,stored", [(8, 24, 32), (16, 16, 32), (5, 8, 16), (33, 16, 64), (64, 0, 64), (1, 48, 64)])
+def test_a_slice_of_the_features(eng, dtype, f, at, stored):
+    """Some of a pixel's features to planes and back, up to the last element of the buffer; the other features stay as they are."""
+    from cldnn_b200 import engine
+    b, y, x = 2, 9, 12
+    rng = np.random.default_rng(10)
+    whole = rng.integers(0, 100, size=(b, y, x, stored)).astype(dtype)
+    p = abi.ReorderParams()
+    p.in_, _ = abi.tensor(abi.dtype_of(whole.dtype), b, f, y, x, "byxf")
+    p.in_.px, p.in_.py, p.in_.pb, p.in_.offset = stored, stored * x, stored * x * y, at
+    p.out, n = abi.tensor(abi.dtype_of(whole.dtype), b, f, y, x, "bfyx")
+    src, dst = eng.upload(whole), eng.upload(np.full(n, 77, dtype=dtype))
+    eng.kernel("reorder_ref").launch(p, engine.make_args(input0=src, output=dst))
+    want = np.ascontiguousarray(whole[..., at:at + f].transpose(0, 3, 1, 2))
+    assert np.array_equal(dst.read(dtype), want.reshape(-1))
+    q = abi.ReorderParams()
+    q.in_, q.out = p.out, p.in_
+    other = rng.integers(100, 120, size=whole.shape).astype(dtype)
+    back = eng.upload(other)
+    eng.kernel("reorder_ref").launch(q, engine.make_args(input0=dst, output=back))
+    other[..., at:at + f] = whole[..., at:at + f]
+    assert np.array_equal(back.read(dtype).reshape(whole.shape), other)
