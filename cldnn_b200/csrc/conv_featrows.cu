@@ -293,7 +293,7 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
                     fv[j] = epi_quant(c, (int32_t)sv[j] + bi[j], qv[j], bf[j], cv[j], el, ev[j]);
                     iv[j] = c.out_dtype == CLDNN_B200_U8 ? sat_i32_from_float(fv[j], 0, 255) : sat_i32_from_float(fv[j], -128, 127);
                 }
-                if (nf == 4 && is_int8(c.out_dtype) && (o & 3) == 0)
+                if (nf == 4 && is_int8(c.out_dtype) && ((reinterpret_cast<uintptr_t>(P.out) + (uintptr_t)o) & 3) == 0)
                     *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(P.out) + o) =
                         (uint32_t)(iv[0] & 0xff) | ((uint32_t)(iv[1] & 0xff) << 8) | ((uint32_t)(iv[2] & 0xff) << 16) | ((uint32_t)(iv[3] & 0xff) << 24);
                 else for (int j = 0; j < nf; ++j) store_sat_float(P.out, c.out_dtype, o + j, fv[j]);

@@ -723,6 +723,8 @@ static int32_t tc_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_par
         if (boxed) return true;
         return sx == 1 && sy == 1 && pixel_dense(t);
     };
+    // (the direct stores of the conversion-free epilogue are vectors too)
+    if (((uintptr_t)a->output & 15) || (p.fused_eltw && ((uintptr_t)P.eltw & 15))) P.fast_epi = P.lean = 0;
     P.staged = (P.fast_epi && tma_ok(p.out, a->output, 1, 1) && (!p.fused_eltw || tma_ok(et, P.eltw, esx, esy))) ? 1 : 0;
     if (p.fused_eltw && !p.in_out_opt && (et.b != p.out.b || (et.y + esy - 1) / esy < p.out.y || (et.x + esx - 1) / esx < p.out.x || et.f < p.ofm)) P.staged = 0;
     P.cw = pl.bn < 128 ? pl.bn : 128; P.col_blocks = pl.bn / P.cw;

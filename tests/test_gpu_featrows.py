@@ -77,3 +77,32 @@ def test_untuned_inner_products(eng, images):
     want, got = cases.run_oracle(case).astype(np.float32), cases.run_gpu(eng, case, "conv_f16_tc", 0).astype(np.float32)
     n = case.out_elems
     assert np.abs(got[:n] - want[:n]).max() <= F16_TOL * np.abs(want[:n]).max()
+
+
+@pytest.mark.parametrize("shift", [1, 2, 7])
+@pytest.mark.parametrize("fused", [False, True])
+def test_8bit_buffers_off_the_vector_alignment(eng, shift, fused):
+    """Output and residual that start anywhere: whole vectors of features have to be stored by bytes, in this form and in the pixel-row kernel."""
+    from cldnn_b200 import engine
+    for geom, order in ((dict(N=3, C=64, K=131, H=7, W=7), abi.EPILOGUE_REF), (dict(N=2, C=160, K=128, H=9, W=11), abi.EPILOGUE_REF),
+                        (dict(N=2, C=64, K=64, H=7, W=7, bias="f32", calib=True, eltw_calib=fused), abi.EPILOGUE_IMAD)):
+        case = cases.make_conv_case(75, out_dtype=np.int8, fused=fused, **geom)
+        case.p.epilogue_order = order
+        want, n = cases.run_oracle(case), case.out_elems
+        bufs = {k: eng.upload(v) for k, v in dict(weights=case.w, bias=case.bias, quant=case.quant, calib=case.calib, eltw_calib=case.ecal).items() if v is not None}
+        src, k, ran = eng.upload(case.inp), eng.kernel("conv_i8_tc"), 0
+        res = eng.upload(np.concatenate([np.zeros(shift, np.int8), case.eltw])) if fused else None
+        for tune in [0, 2, 6, 10, 14, 18, 22] + list(range(I8_BASE, I8_BASE + VARIANTS)):
+            p = cases.copy_params(case.p)
+            p.tune = tune
+            if not k.supports(p):
+                continue
+            out = eng.upload(np.full(n + shift, 77, np.int8))
+            k.launch(p, engine.make_args(input0=src, input1=res.ptr + shift if fused else None, output=out.ptr + shift, **bufs))
+            eng.sync()
+            got = out.read(np.int8)
+            assert eng.device_status() == 0 and (got[:shift] == 77).all()
+            logical = cases.logical_out(case, got[shift:])
+            assert np.array_equal(logical, cases.logical_out(case, want)), "tune %d" % tune
+            ran += 1
+        assert ran >= 10
