@@ -251,7 +251,8 @@ struct node {
     // fused activations (prepare_primitive_fusing)
     int32_t act = CLDNN_B200_ACT_NONE; float act_m = 0.f, act_n = 0.f;
     int32_t eltw_act = CLDNN_B200_ACT_NONE; float eltw_m = 0.f, eltw_n = 0.f;
-    int32_t lrn_size = 0; float lrn_k = 0.f, lrn_alpha = 0.f, lrn_beta = 0.f;   // pooling: the LRN folded in front of it
+    node* lrn = nullptr;                // pooling: the LRN in front of it that its launch computes as well
+    bool absorbed = false;              // lrn: computed inside its pooling's launch, without memory of its own
     // execution
     memory mem;                         // output memory
     memory packed_weights;              // weights re-laid for the chosen kernel
@@ -316,6 +317,10 @@ public:
     void fuse_activations();
     void fuse_conv_eltwise();
     void fuse_lrn_pool();
+    void compute_apart(node* l);
+    bool forced_kernel(const std::string& id, std::string& kernel) const;
+    cldnn_b200_pool_params pool_params(node* n);
+    cldnn_b200_lrn_pool_params lrn_pool_params(node* n, node* l);
     void select_layouts();
     void conv_eltw_read_write_opt();
     void replace_dep(node* consumer, node* from, node* to) { for (auto& id : consumer->p.input) if (id == from->p.id) id = to->p.id; }
@@ -458,26 +463,84 @@ void network_impl::fuse_activations()
     sort(); relayout();
 }
 
-// LRN whose only reader is a 3x3 stride-2 maximum: one launch for both (lrn_pool_f16_byxf).
+// What build_option force_kernel ("<primitive id>=<kernel>[:tune],...") says about a primitive; false: nothing.
+bool network_impl::forced_kernel(const std::string& id, std::string& kernel) const
+{
+    std::stringstream ss(opts.force_kernel); std::string item;
+    while (std::getline(ss, item, ',')) {
+        const size_t eq = item.find('=');
+        if (eq != std::string::npos && item.substr(0, eq) == id) { kernel = item.substr(eq + 1); return true; }
+    }
+    return false;
+}
+
+cldnn_b200_pool_params network_impl::pool_params(node* n)
+{
+    const primitive& p = n->p;
+    const layout& in = n->deps[0]->out;
+    cldnn_b200_pool_params pp{};
+    pp.in = in.desc(); pp.out = n->out.desc();
+    pp.size_x = p.global_pooling ? in.size.x : p.size.x; pp.size_y = p.global_pooling ? in.size.y : p.size.y;
+    pp.stride_x = p.global_pooling ? 1 : p.stride.x; pp.stride_y = p.global_pooling ? 1 : p.stride.y;
+    pp.pad_x = std::max(-p.input_offset.x, 0); pp.pad_y = std::max(-p.input_offset.y, 0);
+    pp.mode = p.pool_mode == pooling_mode::max ? CLDNN_B200_POOL_MAX : CLDNN_B200_POOL_AVG;
+    // pooling_gpu::create, src/gpu/pooling_gpu.cpp:122-130: when the last window runs past input + padding the
+    // average divides by the clipped window
+    const bool dyn = ((n->out.size.x - 1) * pp.stride_x + pp.size_x) > 2 * pp.pad_x + in.size.x ||
+                     ((n->out.size.y - 1) * pp.stride_y + pp.size_y) > 2 * pp.pad_y + in.size.y;
+    if (p.pool_mode == pooling_mode::average && dyn) pp.div_mode = CLDNN_B200_DIV_DYNAMIC_WITH_PADDING;
+    else pp.div_mode = p.pool_mode == pooling_mode::average_no_padding ? CLDNN_B200_DIV_DYNAMIC : CLDNN_B200_DIV_FIXED;
+    pp.act = n->act; pp.act_m = n->act_m; pp.act_n = n->act_n;
+    return pp;
+}
+cldnn_b200_lrn_pool_params network_impl::lrn_pool_params(node* n, node* l)
+{
+    cldnn_b200_lrn_pool_params fp{};
+    fp.pool = pool_params(n); fp.pool.in = l->deps[0]->out.desc();
+    fp.lrn_size = (int32_t)l->p.lrn_size; fp.lrn_k = l->p.lrn_k; fp.lrn_alpha = l->p.lrn_alpha; fp.lrn_beta = l->p.lrn_beta;
+    return fp;
+}
+
+// LRN whose only reader is a pooling that one kernel computes together with it (lrn_pool_f16_byxf): one launch for both, in the layouts
+// chosen before and unless a kernel is forced on either.  The LRN stays in the graph, so that its result can still be asked for
+// (compute_apart): its input keeps its buffer for that, which rules out inputs that the caller or an in-place sum may rewrite.
 void network_impl::fuse_lrn_pool()
 {
-    for (size_t i = 0; i < nodes.size(); ++i) {
-        node* n = nodes[i].get();
-        if (n->removed || n->p.type != "pooling" || n->deps.size() != 1 || n->lrn_size || n->act != CLDNN_B200_ACT_NONE) continue;
+    const char* joint = "lrn_pool_f16_byxf";
+    for (node* n : order) {
+        if (n->p.type != "pooling" || n->deps.size() != 1) continue;
         node* l = n->deps[0];
-        if (l->p.type != "lrn" || l->users.size() != 1 || l->param_uses || l->is_output || l->deps.size() != 1 || l->deps[0]->out.data_type != data_types::f16) continue;
-        const bool window = n->p.pool_mode == pooling_mode::max && !n->p.global_pooling && n->p.size.x == 3 && n->p.size.y == 3 && n->p.stride.x == 2 &&
-                            n->p.stride.y == 2 && n->p.input_offset.x == 0 && n->p.input_offset.y == 0;
-        const tensor& ls = l->out.size; const tensor& os = n->out.size;
-        if (!window || l->p.lrn_size != 5 || ls.feature % 8 || ls.feature > 2048 || 2 * os.x + 1 > ls.x || 2 * os.y + 1 > ls.y) continue;
-        if ((size_t)3 * ls.x * ls.feature * 2 > 64 * 1024 || ls.batch > 65535) continue;          // the kernel's three rows in shared memory
-        n->lrn_size = (int32_t)l->p.lrn_size; n->lrn_k = l->p.lrn_k; n->lrn_alpha = l->p.lrn_alpha; n->lrn_beta = l->p.lrn_beta;
-        n->p.input[0] = l->deps[0]->p.id;
+        if (l->p.type != "lrn" || l->users.size() != 1 || l->param_uses || l->is_output || l->deps.size() != 1) continue;
+        node* d = l->deps[0];
+        if (d->constant() || d->p.type == "input_layout") continue;
+        bool rewritten = false;
+        for (node* u : d->users) rewritten |= u->in_place && u->deps[1] == d;
+        std::string forced;
+        if (rewritten || forced_kernel(l->p.id, forced) || (forced_kernel(n->p.id, forced) && forced != joint)) continue;
+        cldnn_b200_lrn_pool_params fp = lrn_pool_params(n, l);
+        int32_t yes = 0;
+        if (cldnn_b200_kernel_supports(eng->kernel(joint), &fp, sizeof(fp), &yes) != CLDNN_B200_SUCCESS || !yes) continue;
+        n->lrn = l; l->absorbed = true;
         n->fused_ids += (n->fused_ids.empty() ? "" : ",") + l->p.id;
-        l->removed = true;
-        link();
     }
-    sort(); relayout();
+}
+
+// The result of an LRN that is computed inside its pooling's launch has been asked for: it gets memory and a launch of its own from the next
+// pass on, and its values of the last pass now.
+void network_impl::compute_apart(node* l)
+{
+    node* n = l->users[0];
+    const size_t at = n->fused_ids.rfind(l->p.id);
+    n->fused_ids.erase(at > 0 ? at - 1 : 0, l->p.id.size() + (at > 0 ? 1 : 0));
+    n->lrn = nullptr; l->absorbed = false;
+    l->mem = memory(); l->mem.impl = std::make_shared<memory_impl>(); l->mem.impl->l = l->out;
+    l->mem.impl->blk = new_block(eng, std::max<size_t>(l->out.bytes_count(), 16)); pool_bytes += l->mem.impl->blk->bytes;
+    if (n->prepared) {
+        prepare_kernel(l);
+        run_prepared(l);
+        check(cldnn_b200_ctx_sync(eng->ctx), "sync");
+    }
+    inputs_changed = true;
 }
 
 // prepare_conv_eltw_fusing::fuse_conv_eltwise, src/graph_optimizer/prepare_primitive_fusing.cpp:181-337:
@@ -783,16 +846,13 @@ void network_impl::save_cache()
 void network_impl::pick_kernel(node* n, const std::vector<std::string>& candidates, void* params, size_t psize, const void* key_params,
                                const cldnn_b200_args& args, const std::function<void(int)>& set_tune, bool time_all)
 {
-    if (!opts.force_kernel.empty()) {                               // "<primitive id>=<kernel>[:tune],..."
-        std::stringstream ss(opts.force_kernel); std::string item;
-        while (std::getline(ss, item, ',')) {
-            const size_t eq = item.find('='); if (eq == std::string::npos || item.substr(0, eq) != n->p.id) continue;
-            std::string k = item.substr(eq + 1); int tune = 0; const size_t colon = k.find(':');
-            if (colon != std::string::npos) { tune = std::atoi(k.substr(colon + 1).c_str()); k = k.substr(0, colon); }
-            bool known = false; for (auto& c : candidates) known |= c == k;
-            if (!known) throw error(n->p.id + ": forced kernel '" + k + "' does not implement " + n->p.type, CLDNN_B200_INVALID_ARG);
-            n->kernel = k; n->tune = tune; set_tune(tune); return;
-        }
+    std::string k;
+    if (forced_kernel(n->p.id, k)) {
+        int tune = 0; const size_t colon = k.find(':');
+        if (colon != std::string::npos) { tune = std::atoi(k.substr(colon + 1).c_str()); k = k.substr(0, colon); }
+        bool known = false; for (auto& c : candidates) known |= c == k;
+        if (!known) throw error(n->p.id + ": forced kernel '" + k + "' does not implement " + n->p.type, CLDNN_B200_INVALID_ARG);
+        n->kernel = k; n->tune = tune; set_tune(tune); return;
     }
     set_tune(0);
     // the key carries the generation of the kernel set: timings taken on older kernels must not be reused.  `key_params`:
@@ -880,7 +940,7 @@ void network_impl::prepare_kernel(node* n)
     const primitive& p = n->p;
     const std::string& t = p.type;
     cldnn_b200_args a{};
-    if (!n->deps.empty()) a.input0 = n->deps[0]->mem.device_ptr();
+    if (!n->deps.empty()) a.input0 = (n->lrn ? n->lrn : n)->deps[0]->mem.device_ptr();
     if (n->deps.size() > 1) a.input1 = n->deps[1]->mem.device_ptr();
     a.output = n->mem.device_ptr();
     if (n->weights) a.weights = n->weights->mem.device_ptr();
@@ -1069,45 +1129,12 @@ void network_impl::prepare_kernel(node* n)
         return;
     }
     if (t == "pooling") {
-        const layout& in = n->deps[0]->out;
-        cldnn_b200_pool_params pp{};
-        pp.in = in.desc(); pp.out = n->out.desc();
-        pp.size_x = p.global_pooling ? in.size.x : p.size.x; pp.size_y = p.global_pooling ? in.size.y : p.size.y;
-        pp.stride_x = p.global_pooling ? 1 : p.stride.x; pp.stride_y = p.global_pooling ? 1 : p.stride.y;
-        pp.pad_x = std::max(-p.input_offset.x, 0); pp.pad_y = std::max(-p.input_offset.y, 0);
-        pp.mode = p.pool_mode == pooling_mode::max ? CLDNN_B200_POOL_MAX : CLDNN_B200_POOL_AVG;
-        // pooling_gpu::create, src/gpu/pooling_gpu.cpp:122-130: when the last window runs past input + padding the
-        // average divides by the clipped window
-        const bool dyn = ((n->out.size.x - 1) * pp.stride_x + pp.size_x) > 2 * pp.pad_x + in.size.x ||
-                         ((n->out.size.y - 1) * pp.stride_y + pp.size_y) > 2 * pp.pad_y + in.size.y;
-        if (p.pool_mode == pooling_mode::average && dyn) pp.div_mode = CLDNN_B200_DIV_DYNAMIC_WITH_PADDING;
-        else pp.div_mode = p.pool_mode == pooling_mode::average_no_padding ? CLDNN_B200_DIV_DYNAMIC : CLDNN_B200_DIV_FIXED;
-        pp.act = n->act; pp.act_m = n->act_m; pp.act_n = n->act_n;
-        if (n->lrn_size) {
-            cldnn_b200_lrn_pool_params fp{}; fp.pool = pp;
-            fp.lrn_size = n->lrn_size; fp.lrn_k = n->lrn_k; fp.lrn_alpha = n->lrn_alpha; fp.lrn_beta = n->lrn_beta;
-            int32_t yes = 0;
-            if (cldnn_b200_kernel_supports(eng->kernel("lrn_pool_f16_byxf"), &fp, sizeof(fp), &yes) == CLDNN_B200_SUCCESS && yes) {
-                finish({"lrn_pool_f16_byxf"}, &fp, sizeof(fp), [](int) {});
-                return;
-            }
-            // a layout the joint kernel does not take: the two launches, with the normalised map in a workspace
-            n->scratch = new_block(eng, in.bytes_count());
-            cldnn_b200_lrn_params lp{}; lp.in = lp.out = in.desc();
-            lp.size = n->lrn_size; lp.k = n->lrn_k; lp.alpha = n->lrn_alpha; lp.beta = n->lrn_beta;
-            cldnn_b200_args la = a; la.output = n->scratch->dev; a.input0 = n->scratch->dev;
-            auto first_of = [&](const std::vector<std::string>& cands, const void* params, size_t size) {
-                for (auto& c : cands) if (cldnn_b200_kernel_supports(eng->kernel(c), params, size, &yes) == CLDNN_B200_SUCCESS && yes) return c;
-                throw error(p.id + ": cannot find a proper kernel with these arguments", CLDNN_B200_ERROR);
-            };
-            cldnn_b200_prepared second = nullptr;
-            const std::string lk = first_of({"lrn_f16_byxf", "lrn_ref"}, &lp, sizeof(lp));
-            n->kernel = first_of({"pooling_f16_byxf", "pooling_ref"}, &pp, sizeof(pp)); n->tune = 0;
-            check(cldnn_b200_prepare(eng->kernel(lk), &lp, sizeof(lp), &la, &n->prepared), p.id + " (" + lk + ")");
-            check(cldnn_b200_prepare(eng->kernel(n->kernel), &pp, sizeof(pp), &a, &second), p.id + " (" + n->kernel + ")");
-            n->more_prepared.push_back(second);
+        if (n->lrn) {
+            cldnn_b200_lrn_pool_params fp = lrn_pool_params(n, n->lrn);
+            finish({"lrn_pool_f16_byxf"}, &fp, sizeof(fp), [](int) {});
             return;
         }
+        cldnn_b200_pool_params pp = pool_params(n);
         finish({"pooling_i8_byxf", "pooling_f16_byxf", "pooling_ref"}, &pp, sizeof(pp), [](int) {});
         return;
     }
@@ -1185,12 +1212,13 @@ void network_impl::allocate_and_prepare()
         for (node* d : n->deps) last_use[d->order] = std::max(last_use[d->order], n->order);
         for (node* d : n->params()) last_use[d->order] = std::max(last_use[d->order], n->order);   // a bias may be computed by the network
         if (n->is_output) last_use[n->order] = 1 << 30;
+        if (n->absorbed) last_use[n->deps[0]->order] = 1 << 30;
     }
     std::multimap<size_t, std::shared_ptr<block>> free_blocks;
     std::vector<std::pair<int, std::shared_ptr<block>>> live;       // (last use, block)
     for (node* n : order) {
         if (n->p.type == "data") { n->mem = n->p.mem; continue; }
-        if (n->p.type == "input_layout") continue;                  // bound by set_input_data
+        if (n->p.type == "input_layout" || n->absorbed) continue;    // bound by set_input_data; part of another launch
         if (n->in_place) {
             // the second input's buffer becomes the output: it now lives until this node's last reader
             node* r = n->deps[1];
@@ -1234,9 +1262,9 @@ void network_impl::build(const topology& topo)
         fuse_activations();
         fuse_conv_eltwise();
         fuse_activations();                                         // relu behind a freshly fused conv+eltwise
-        fuse_lrn_pool();
         select_layouts();
         if (opts.conv_eltw_read_write_opt) conv_eltw_read_write_opt();
+        fuse_lrn_pool();
     }
     load_cache();
     allocate_and_prepare();
@@ -1253,7 +1281,7 @@ void network_impl::execute()
             for (auto pr : n->more_prepared) cldnn_b200_prepared_destroy(pr);
             n->more_prepared.clear();
         }
-        for (node* n : order) if (n->p.type != "data" && n->p.type != "input_layout") prepare_kernel(n);
+        for (node* n : order) if (n->p.type != "data" && n->p.type != "input_layout" && !n->absorbed) prepare_kernel(n);
         save_cache();
         check(cldnn_b200_ctx_sync(eng->ctx), "sync");
         launches = 0; for (node* n : order) if (n->prepared) launches += 1 + n->more_prepared.size();
@@ -1310,6 +1338,7 @@ memory network::output_memory(const std::string& id) const
 {
     for (node* n : impl->order) if (n->is_output && (n->answers_for == id || n->p.id == id)) return n->mem;
     node* n = impl->get(id);
+    if (n->absorbed) impl->compute_apart(n);
     if (!n->mem) throw error("primitive '" + id + "' has no memory (fused away); request it as an output", CLDNN_B200_INVALID_ARG);
     return n->mem;
 }
@@ -1318,6 +1347,7 @@ std::vector<primitive_info> network::get_primitives_info() const
 {
     std::vector<primitive_info> v;
     for (node* n : impl->order) {
+        if (n->absorbed) continue;
         primitive_info i; i.id = n->p.id; i.type = n->p.type; i.original_ids = n->fused_ids; i.kernel = n->kernel; i.tune = n->tune; i.output = n->out; i.is_output = n->is_output; i.in_place = n->in_place;
         v.push_back(i);
     }

@@ -64,6 +64,71 @@ def test_network_on_a_planar_map(features):
         net.set_input_data("input", cl.memory.from_numpy(eng, x))
         net.execute()
         got.append(net.get_output("pool").to_numpy().astype(np.float32))
+        assert _kernels(net) == {"input": "", "norm": "lrn_ref", "pool": "pooling_ref"}
         net.execute()
         assert np.array_equal(net.get_output("pool").to_numpy().astype(np.float32), got[-1])
     assert got[0].shape == got[1].shape and np.abs(got[0] - got[1]).max() <= 2e-3 * np.abs(got[0]).max()
+
+
+def _build(eng, images, size, outputs, **options):
+    """convolution -> LRN -> 3x3 stride-2 maximum -> convolution -> convolution, with intermediate buffers that are reused."""
+    from cldnn_b200 import cldnn as cl
+    rng, dt = np.random.default_rng(33), cl.data_types
+    weights = {"w1": (32, 16, 3, 3), "w2": (64, 32, 3, 3), "w3": (256, 64, 3, 3)}
+    mems = {n: cl.memory.from_numpy(eng, (rng.standard_normal(s) / np.sqrt(np.prod(s[1:]))).astype(np.float16)) for n, s in weights.items()}
+    lay = cl.layout(dt.f16, cl.format.bfyx, cl.tensor(images, 16, size, size))
+    x = (rng.standard_normal((images, 16, size, size)) * 4).astype(np.float16)
+    prims = [cl.input_layout("input", lay)] + [cl.data(n, m) for n, m in mems.items()] + [
+        cl.convolution("conv1", "input", "w1", input_offset=(-1, -1), with_activation=True), cl.lrn("norm1", "conv1", alpha=1e-2),
+        cl.pooling("pool1", "norm1", cl.pooling_mode.max, size=(3, 3), stride=(2, 2)), cl.convolution("conv2", "pool1", "w2", input_offset=(-1, -1)),
+        cl.convolution("conv3", "conv2", "w3", input_offset=(-1, -1))]
+    net = cl.network(eng, cl.topology(*prims), cl.build_options(optimize_data=True, outputs=outputs, **options))
+    inp = cl.memory.from_numpy(eng, x)
+    net.set_input_data("input", inp)
+    return net, inp, x
+
+
+def _kernels(net):
+    return {i["id"]: i["kernel"] for i in net.primitives_info()}
+
+
+def test_forced_kernels_keep_the_two_launches(tmp_path):
+    from cldnn_b200 import cldnn as cl
+    eng = cl.engine(0)
+    got = {}
+    for forced in (None, "pool1=lrn_pool_f16_byxf", "pool1=pooling_f16_byxf", "pool1=pooling_ref", "norm1=lrn_f16_byxf", "norm1=lrn_ref"):
+        net, inp, _ = _build(eng, 3, 21, ["conv3", "pool1"], force_kernel=forced)
+        net.execute()
+        got[forced], k = net.get_output("pool1").to_numpy(), _kernels(net)
+        apart = forced is not None and forced != "pool1=lrn_pool_f16_byxf"
+        assert ("norm1" in k) == apart and (k["pool1"] == "lrn_pool_f16_byxf") != apart
+        if apart:
+            assert k[forced.split("=")[0]] == forced.split("=")[1]
+    for forced in list(got)[:5]:
+        assert np.array_equal(got[forced], got[None]), forced
+    scale = np.abs(got[None].astype(np.float32)).max()
+    assert np.abs(got["norm1=lrn_ref"].astype(np.float32) - got[None].astype(np.float32)).max() <= 2e-3 * scale
+    net, inp, _ = _build(eng, 3, 21, ["conv3"], tuning=cl.tuning_mode.tuning_tune_and_cache, tuning_cache_path=str(tmp_path / "cache.json"))
+    net.execute()
+    assert _kernels(net)["pool1"] == "lrn_pool_f16_byxf"
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("before", [False, True])
+def test_the_normalised_map_can_be_asked_for(graph, before):
+    """get_output of the LRN that runs inside the pooling's launch: its values of that pass, and again after the next one with other input."""
+    from cldnn_b200 import cldnn as cl
+    eng = cl.engine(0)
+    apart, inp_a, x = _build(eng, 2, 19, ["conv3", "norm1"], use_graph=graph)
+    net, inp, _ = _build(eng, 2, 19, ["conv3"], use_graph=graph)
+    norm = net.get_output("norm1") if before else None
+    for scale in (1, 2, -1):
+        for n, m in ((apart, inp_a), (net, inp)):
+            m.set_values((x * scale).astype(np.float16))
+            n.execute()
+        assert before or scale != 1 or "norm1" not in _kernels(net)
+        norm = norm or net.get_output("norm1")
+        net.wait()
+        assert np.array_equal(norm.to_numpy(), apart.get_output("norm1").to_numpy())
+        assert np.array_equal(net.get_output("conv3").to_numpy(), apart.get_output("conv3").to_numpy())
+    assert _kernels(net)["norm1"] == "lrn_f16_byxf" and _kernels(net)["pool1"] == "pooling_f16_byxf"
