@@ -50,7 +50,7 @@ constexpr uint32_t kErr = 0x60u;
 enum AMode { A_FLAT = 0, A_IM2COL = 1, A_TILED = 2, A_PATCH = 3 };
 
 struct alignas(64) Params {
-    CUtensorMap tmA, tmB, tmO, tmE;
+    CUtensorMap tmA[kGroupMaps], tmB, tmO, tmE;   // activations: [0], or one per group (group_maps)
     int32_t a_mode;
     int32_t N, P, Q;
     int32_t kh, kw, stride_x, stride_y, pad_x, pad_y, dil_x, dil_y;
@@ -66,6 +66,7 @@ struct alignas(64) Params {
     int32_t early_params;                    // weights may be read before the previous kernel has ended
     int32_t pair;                            // CTA pairs: m_tiles is even, the weight box holds bn / 2 rows
     int32_t group_tiles, group_ch;           // grouped: feature tiles per group (0: one group), its input features
+    int32_t group_maps;                      // grouped, slices that end inside a chunk: a tensor map per group
     float act_m, act_n, eltw_m, eltw_n;
     const void* bias;
     uint32_t* status;
@@ -191,7 +192,7 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
         mbar_init(smem_u32(&aux->b_full), 1); mbar_init(smem_u32(&aux->drain), 1);
         aux->abort = 0u;
         mbar_fence_init();
-        prefetch_tensormap(&P.tmA); prefetch_tensormap(&P.tmB); prefetch_tensormap(&P.tmO);
+        prefetch_tensormap(&P.tmA[0]); prefetch_tensormap(&P.tmB); prefetch_tensormap(&P.tmO);
         if (kFused) prefetch_tensormap(&P.tmE);
     }
     if (warp == 1) {
@@ -239,7 +240,8 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
                     const int tw = m_tile % P.tiles_w; const int t2 = m_tile / P.tiles_w;
                     c_w = tw * P.bw - P.pad_x; c_h = (t2 % P.tiles_h) * P.bh - P.pad_y; c_n = (t2 / P.tiles_h) * P.bb;
                 }
-                const int g0 = P.group_tiles ? n_tile / P.group_tiles * P.group_ch : 0;      // first input feature of the tile's group
+                const int group = P.group_tiles ? n_tile / P.group_tiles : 0, g0 = group * P.group_ch;   // first input feature of the tile's group
+                const CUtensorMap* ta = P.tmA + (P.group_maps ? group : 0);
                 int tap = P.batch_tiles ? m_tile / P.batch_tiles : 0, cc = 0, r = 0, s = 0;
                 for (int ks = 0; ks < P.k_steps; ++ks) {
                     if (!__all_sync(0xffffffffu, mbar_wait_lean(smem_u32(&aux->empty[stage]), phase ^ 1u, s_abort, P.status, kErr))) { ok = false; break; }
@@ -249,20 +251,20 @@ conv_f16_tc_kernel(const __grid_constant__ Params P)
                     const int c0 = cc * bke, a0 = g0 + c0;
                     if (leader && patch) {
                         mbar_expect_tx(full, (uint32_t)P.a_tx_bytes);
-                        for (int sc = 0; sc < P.kw; ++sc) tma_load_4d(a_dst + (uint32_t)(sc * P.patch_alloc), &P.tmA, full, c0, c_w + sc, c_h, c_n);
+                        for (int sc = 0; sc < P.kw; ++sc) tma_load_4d(a_dst + (uint32_t)(sc * P.patch_alloc), ta, full, c0, c_w + sc, c_h, c_n);
                     } else if (leader && kPair) {
                         // both CTAs' copies report to rank 0's barrier, which expects the bytes of both
                         const uint32_t full_r0 = mapa_rank(full, 0u);
                         if (rank == 0u) mbar_expect_tx(full, 2u * (uint32_t)(P.a_tx_bytes + P.b_tx_bytes));
-                        if (P.a_mode == A_FLAT) tma_load_2d_pair(a_dst, &P.tmA, full_r0, a0, m_tile * kBM);
-                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d_pair(a_dst, &P.tmA, full_r0, a0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
-                        else tma_load_4d_pair(a_dst, &P.tmA, full_r0, a0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
+                        if (P.a_mode == A_FLAT) tma_load_2d_pair(a_dst, ta, full_r0, a0, m_tile * kBM);
+                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d_pair(a_dst, ta, full_r0, a0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
+                        else tma_load_4d_pair(a_dst, ta, full_r0, a0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
                         tma_load_3d_pair(b_dst, &P.tmB, full_r0, c0, tap, n_tile * BN + (int)rank * (BN / 2));
                     } else if (leader) {
                         mbar_expect_tx(full, (uint32_t)(P.a_tx_bytes + P.b_tx_bytes));
-                        if (P.a_mode == A_FLAT) tma_load_2d(a_dst, &P.tmA, full, a0, m_tile * kBM);
-                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d(a_dst, &P.tmA, full, a0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
-                        else tma_load_4d(a_dst, &P.tmA, full, a0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
+                        if (P.a_mode == A_FLAT) tma_load_2d(a_dst, ta, full, a0, m_tile * kBM);
+                        else if (P.a_mode == A_IM2COL) tma_load_im2col_4d(a_dst, ta, full, a0, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
+                        else tma_load_4d(a_dst, ta, full, a0, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
                         tma_load_3d(b_dst, &P.tmB, full, c0, tap, n_tile * BN);
                     }
                     ++issued;
@@ -737,7 +739,6 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;
     P.kh = p.kh; P.kw = p.kw; P.stride_x = p.stride_x; P.stride_y = p.stride_y; P.pad_x = p.pad_x; P.pad_y = p.pad_y; P.dil_x = p.dil_x; P.dil_y = p.dil_y;
     const int cs = (int)reduction_features(p);
-    const cuuint64_t a_features = (cuuint64_t)p.in.px;               // of the activations' tensor map
     const int bke = pl.bk / 2;
     P.bk = pl.bk; P.chunks = cs / bke; P.k_steps = p.kh * p.kw * P.chunks;
     P.bn = pl.bn; P.n_tiles = (p.ofm + pl.bn - 1) / pl.bn;
@@ -774,7 +775,7 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     P.idesc = (1u << 4) | ((uint32_t)(pl.bn >> 3) << 17) | ((uint32_t)((pl.pair ? 2 * f16tc::kBM : f16tc::kBM) >> 4) << 24);
     const int nbuf = pl.bn >= 256 ? 2 : 4;
     P.tmem_cols = (uint32_t)(nbuf * pl.bn);
-    if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / pl.bn; P.group_ch = p.ifm; }
+    if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / pl.bn; P.group_ch = p.ifm; P.group_maps = slices_overhang(p); }
     P.ofm = p.ofm; P.fused = p.fused_eltw; P.bias_dtype = p.bias_dtype; P.act = p.act; P.eltw_act = p.eltw_act;
     P.act_m = p.act_m; P.act_n = p.act_n; P.eltw_m = p.eltw_m; P.eltw_n = p.eltw_n;
     P.bias = a->bias; P.status = ctx->d_status;
@@ -798,39 +799,44 @@ static int32_t f16_prepare_as(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_pa
     const CUtensorMapSwizzle sw = pl.bk == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (pl.bk == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     void* in_ptr = (char*)const_cast<void*>(a->input0) + p.in.offset * 2;
     CUresult cr;
-    if (pl.a_mode == f16tc::A_FLAT) {
-        cuuint64_t dims[2] = {a_features, (cuuint64_t)P.M_total};
-        cuuint64_t strides[1] = {(cuuint64_t)(p.in.px * 2)};
-        cuuint32_t box[2] = {(cuuint32_t)bke, (cuuint32_t)f16tc::kBM};
-        cuuint32_t es[2] = {1, 1};
-        cr = h_encode_tiled(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else if (pl.a_mode == f16tc::A_IM2COL) {
-        cuuint64_t dims[4] = {a_features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
-        cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * 2), (cuuint64_t)(p.in.py * 2), (cuuint64_t)(p.in.pb * 2)};
-        int lower[2] = {-p.pad_x, -p.pad_y};
-        int upper[2] = {p.pad_x - (p.kw - 1) * p.dil_x, p.pad_y - (p.kh - 1) * p.dil_y};
-        cuuint32_t es[4] = {1, (cuuint32_t)p.stride_x, (cuuint32_t)p.stride_y, 1};
-        cr = h_encode_im2col(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in_ptr, dims, strides, lower, upper, (cuuint32_t)bke, (cuuint32_t)f16tc::kBM, es,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else if (patch) {
-        cuuint64_t dims[4] = {a_features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
-        cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * 2), (cuuint64_t)(p.in.py * 2), (cuuint64_t)(p.in.pb * 2)};
-        cuuint32_t box[4] = {(cuuint32_t)bke, (cuuint32_t)pl.bw, (cuuint32_t)(pl.bh + p.kh - 1), 1};
-        cuuint32_t es[4] = {1, 1, 1, 1};
-        cr = h_encode_tiled(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else {
-        const int sx = p.stride_x, sy = p.stride_y;
-        const bool strided_view = sx != 1 || sy != 1;
-        cuuint64_t dims[4] = {a_features, (cuuint64_t)(strided_view ? P.Q : p.in.x), (cuuint64_t)(strided_view ? P.P : p.in.y), (cuuint64_t)p.in.b};
-        cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * sx * 2), (cuuint64_t)(p.in.py * sy * 2), (cuuint64_t)(p.in.pb * 2)};
-        cuuint32_t box[4] = {(cuuint32_t)bke, (cuuint32_t)pl.bw, (cuuint32_t)pl.bh, (cuuint32_t)pl.bb};
-        cuuint32_t es[4] = {1, 1, 1, 1};
-        cr = h_encode_tiled(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-    if (cr != CUDA_SUCCESS) return fail(CLDNN_B200_DEVICE_ERROR, "conv_f16_tc: activation tensor map rejected by the driver (CUresult " + std::to_string((int)cr) + ")");
+    auto encode_a = [&](CUtensorMap* tm, cuuint64_t features) -> int32_t {      // `features`: where the pixels' reduction ends
+        if (pl.a_mode == f16tc::A_FLAT) {
+            cuuint64_t dims[2] = {features, (cuuint64_t)P.M_total};
+            cuuint64_t strides[1] = {(cuuint64_t)(p.in.px * 2)};
+            cuuint32_t box[2] = {(cuuint32_t)bke, (cuuint32_t)f16tc::kBM};
+            cuuint32_t es[2] = {1, 1};
+            cr = h_encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        } else if (pl.a_mode == f16tc::A_IM2COL) {
+            cuuint64_t dims[4] = {features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
+            cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * 2), (cuuint64_t)(p.in.py * 2), (cuuint64_t)(p.in.pb * 2)};
+            int lower[2] = {-p.pad_x, -p.pad_y};
+            int upper[2] = {p.pad_x - (p.kw - 1) * p.dil_x, p.pad_y - (p.kh - 1) * p.dil_y};
+            cuuint32_t es[4] = {1, (cuuint32_t)p.stride_x, (cuuint32_t)p.stride_y, 1};
+            cr = h_encode_im2col(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in_ptr, dims, strides, lower, upper, (cuuint32_t)bke, (cuuint32_t)f16tc::kBM, es,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        } else if (patch) {
+            cuuint64_t dims[4] = {features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
+            cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * 2), (cuuint64_t)(p.in.py * 2), (cuuint64_t)(p.in.pb * 2)};
+            cuuint32_t box[4] = {(cuuint32_t)bke, (cuuint32_t)pl.bw, (cuuint32_t)(pl.bh + p.kh - 1), 1};
+            cuuint32_t es[4] = {1, 1, 1, 1};
+            cr = h_encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        } else {
+            const int sx = p.stride_x, sy = p.stride_y;
+            const bool strided_view = sx != 1 || sy != 1;
+            cuuint64_t dims[4] = {features, (cuuint64_t)(strided_view ? P.Q : p.in.x), (cuuint64_t)(strided_view ? P.P : p.in.y), (cuuint64_t)p.in.b};
+            cuuint64_t strides[3] = {(cuuint64_t)(p.in.px * sx * 2), (cuuint64_t)(p.in.py * sy * 2), (cuuint64_t)(p.in.pb * 2)};
+            cuuint32_t box[4] = {(cuuint32_t)bke, (cuuint32_t)pl.bw, (cuuint32_t)pl.bh, (cuuint32_t)pl.bb};
+            cuuint32_t es[4] = {1, 1, 1, 1};
+            cr = h_encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in_ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        }
+        if (cr != CUDA_SUCCESS) return fail(CLDNN_B200_DEVICE_ERROR, "conv_f16_tc: activation tensor map rejected by the driver (CUresult " + std::to_string((int)cr) + ")");
+        return CLDNN_B200_SUCCESS;
+    };
+    for (int g = 0; g < (P.group_maps ? p.groups : 1); ++g)
+        if (const int32_t st = encode_a(&P.tmA[g], (cuuint64_t)(P.group_maps ? (g + 1) * p.ifm : p.in.px))) return st;
     {
         cuuint64_t dims[3] = {(cuuint64_t)cs, (cuuint64_t)(p.kh * p.kw), (cuuint64_t)p.ofm};
         cuuint64_t strides[2] = {(cuuint64_t)(p.w_px * 2), (cuuint64_t)(p.w_po * 2)};
@@ -904,7 +910,7 @@ int32_t f16_batched_gemm_prepare(cldnn_b200_ctx_impl* ctx, const void* A, const 
     {
         cuuint64_t dims[2] = {(cuuint64_t)cs, (cuuint64_t)P.M_total}; cuuint64_t strides[1] = {(cuuint64_t)cs * 2};
         cuuint32_t box[2] = {(cuuint32_t)bke, (cuuint32_t)f16tc::kBM}; cuuint32_t es[2] = {1, 1};
-        cr = h_encode_tiled(&P.tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(A), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+        cr = h_encode_tiled(&P.tmA[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(A), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (cr == CUDA_SUCCESS) {

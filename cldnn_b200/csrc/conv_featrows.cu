@@ -30,7 +30,7 @@ constexpr uint32_t kFrErr = 0xa0u;
 enum { FR_FLAT = 0, FR_IM2COL = 1, FR_TILED = 2 };
 
 struct alignas(64) FrParams {
-    CUtensorMap tmW, tmX;
+    CUtensorMap tmW, tmX[kGroupMaps];         // activations: [0], or one per group (group_maps)
     int32_t mode, N, P, Q;
     int32_t kw, stride_x, stride_y, pad_x, pad_y, dil_x, dil_y;
     int32_t bk, chunks, k_steps, split;
@@ -42,6 +42,7 @@ struct alignas(64) FrParams {
     int32_t ofm;
     int32_t early_params;                     // weights and per-feature constants may be read before the previous kernel has ended
     int32_t group_tiles, group_ch;            // grouped: feature tiles per group (0: one group), its input features
+    int32_t group_maps;                       // grouped fp16 whose slices end inside a chunk: a tensor map per group
     int64_t out_px, out_py, out_pb, out_off, el_px, el_py, el_pb, el_off;
     int32_t el_sx, el_sy;
     void* out; const void* eltw; const void* bias; const float* quant; const float* calib; const float* ecal;
@@ -129,7 +130,7 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
         mbar_init(smem_u32(&aux->tmem_full), 1);
         aux->abort = 0u;
         mbar_fence_init();
-        prefetch_tensormap(&P.tmW); prefetch_tensormap(&P.tmX);
+        prefetch_tensormap(&P.tmW); prefetch_tensormap(&P.tmX[P.group_maps ? m_tile / P.group_tiles : 0]);
     }
     if (warp == 1) { tmem_alloc(smem_u32(&aux->tmem_base), P.tmem_cols); tmem_relinquish(); }
     tc_fence_before();
@@ -179,7 +180,8 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
             const int tw = n_tile % P.tiles_w, t2 = n_tile / P.tiles_w;
             c_w = tw * P.bw - P.pad_x; c_h = (t2 % P.tiles_h) * P.bh - P.pad_y; c_n = (t2 / P.tiles_h) * P.bb;
         }
-        const int g0 = P.group_tiles ? m_tile / P.group_tiles * P.group_ch : 0;
+        const int group = P.group_tiles ? m_tile / P.group_tiles : 0, g0 = group * P.group_ch;
+        const CUtensorMap* tx = P.tmX + (P.group_maps ? group : 0);
         int r = tap / P.kw, s = tap - r * P.kw;
         int issued = pre; bool ok = true;
         for (int i = 0; i < steps; ++i) {
@@ -191,9 +193,9 @@ conv_featrows_kernel(const __grid_constant__ FrParams P)
             }
             if (leader) {
                 const uint32_t full = smem_u32(&aux->full[st]), dst = b_base + (uint32_t)st * (uint32_t)P.b_stage_bytes;
-                if (P.mode == FR_FLAT) tma_load_2d(dst, &P.tmX, full, g0 + cc * bke, n_tile * P.cols);
-                else if (P.mode == FR_IM2COL) tma_load_im2col_4d(dst, &P.tmX, full, g0 + cc * bke, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
-                else tma_load_4d(dst, &P.tmX, full, g0 + cc * bke, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
+                if (P.mode == FR_FLAT) tma_load_2d(dst, tx, full, g0 + cc * bke, n_tile * P.cols);
+                else if (P.mode == FR_IM2COL) tma_load_im2col_4d(dst, tx, full, g0 + cc * bke, c_w, c_h, c_n, (uint16_t)(s * P.dil_x), (uint16_t)(r * P.dil_y));
+                else tma_load_4d(dst, tx, full, g0 + cc * bke, c_w + s * P.dil_x, c_h + r * P.dil_y, c_n);
             }
             if (++cc == P.chunks) { cc = 0; ++tap; if (++s == P.kw) { s = 0; ++r; } }
         }
@@ -355,7 +357,7 @@ bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::stri
     if (f16 && (p.out.px % 4 || p.out.py % 4 || p.out.pb % 4 || p.out.offset % 4)) return no("the feature-row form stores four features at a time");
     pl.cols = kCols[variant / kFrSplits]; pl.split = 1 << (variant % kFrSplits);
     const int64_t es = f16 ? 2 : 1, cs = reduction_features(p) * es;
-    const int bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32);
+    const int bk = (int)chunk_bytes(cs);
     const int64_t steps = (int64_t)p.kh * p.kw * (cs / bk);
     if (pl.split > steps) return no("fewer reduction steps than CTAs");
     const bool pointwise = p.kh == 1 && p.kw == 1 && p.pad_x == 0 && p.pad_y == 0;
@@ -385,7 +387,7 @@ int fr_inner_product_variant(const cldnn_b200_conv_params& p)
     if (p.groups != 1 || p.kh != 1 || p.kw != 1 || p.in.x != 1 || p.in.y != 1 || p.pad_x || p.pad_y || p.stride_x != 1 || p.stride_y != 1) return -1;
     constexpr int64_t kSMs = 148;
     const int64_t cs = p.in.px * (p.in.dtype == CLDNN_B200_F16 ? 2 : 1), n = p.out.b, m_tiles = (p.ofm + kRows - 1) / kRows;
-    const int64_t steps = cs / (cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32));
+    const int64_t steps = cs / chunk_bytes(cs);
     int ci = 0;                                                      // kCols index: 16, 32, 64, 128
     auto n_tiles = [&](int i) { return (n + kCols[i] - 1) / kCols[i]; };
     auto widest = [&](int i) { int s = kFrSplits - 1; while (s > 0 && (int64_t)(n_tiles(i) > 1 ? 4 : 1) * (1 << s) > steps) --s; return s; };
@@ -408,7 +410,7 @@ double fr_cost(const cldnn_b200_conv_params& p, int& variant)
     const bool f16 = p.in.dtype == CLDNN_B200_F16;
     const Cost& c = f16 ? kF16 : kI8;
     const int64_t cs = reduction_features(p) * (f16 ? 2 : 1), pixels = (int64_t)p.out.b * p.out.y * p.out.x;
-    const int64_t bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32), steps = (int64_t)p.kh * p.kw * (cs / bk), m_tiles = (p.ofm + kRows - 1) / kRows;
+    const int64_t bk = chunk_bytes(cs), steps = (int64_t)p.kh * p.kw * (cs / bk), m_tiles = (p.ofm + kRows - 1) / kRows;
     double best = 0.0;
     for (int v = 0; v < kFrVariants; ++v) {
         FrPlan pl;
@@ -433,7 +435,7 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     P.mode = pl.mode; P.N = p.out.b; P.P = p.out.y; P.Q = p.out.x;
     P.kw = p.kw; P.stride_x = p.stride_x; P.stride_y = p.stride_y; P.pad_x = p.pad_x; P.pad_y = p.pad_y; P.dil_x = p.dil_x; P.dil_y = p.dil_y;
     const int64_t cs = reduction_features(p) * es, xs = p.in.px * es;   // bytes of K per tap, pixel pitch of the activations
-    P.bk = cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32);
+    P.bk = (int)chunk_bytes(cs);
     P.chunks = (int)(cs / P.bk); P.k_steps = p.kh * p.kw * P.chunks; P.split = pl.split;
     P.cols = pl.cols; P.bw = pl.bw; P.bh = pl.bh; P.bb = pl.bb;
     const int64_t pixels = (int64_t)P.N * P.P * P.Q;
@@ -457,7 +459,7 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     P.idesc |= ((uint32_t)(P.cols >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
     P.tmem_cols = (uint32_t)(P.cols < 32 ? 32 : P.cols);
     P.ofm = p.ofm; P.early_params = p.constant_params;
-    if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / kRows; P.group_ch = p.ifm; }
+    if (p.groups > 1) { P.group_tiles = p.ofm / p.groups / kRows; P.group_ch = p.ifm; P.group_maps = slices_overhang(p); }
     const cldnn_b200_tensor& et = p.in_out_opt ? p.out : p.eltw;
     P.out_px = p.out.px; P.out_py = p.out.py; P.out_pb = p.out.pb; P.out_off = p.out.offset;
     if (p.fused_eltw) {
@@ -490,30 +492,35 @@ int32_t fr_prepare(cldnn_b200_ctx_impl* ctx, const cldnn_b200_conv_params& p, co
     const cuuint32_t bke = (cuuint32_t)(P.bk / es);
     void* in_ptr = (char*)const_cast<void*>(a->input0) + p.in.offset * es;
     CUresult cr;
-    if (pl.mode == FR_FLAT) {
-        cuuint64_t dims[2] = {(cuuint64_t)p.in.px, (cuuint64_t)P.M_total}; cuuint64_t strides[1] = {(cuuint64_t)xs};
-        cuuint32_t box[2] = {bke, (cuuint32_t)P.cols}; cuuint32_t one[2] = {1, 1};
-        cr = fr_encode_tiled(&P.tmX, dt, 2, in_ptr, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else if (pl.mode == FR_IM2COL) {
-        cuuint64_t dims[4] = {(cuuint64_t)p.in.px, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
-        cuuint64_t strides[3] = {(cuuint64_t)xs, (cuuint64_t)(p.in.py * es), (cuuint64_t)(p.in.pb * es)};
-        int lower[2] = {-p.pad_x, -p.pad_y};
-        int upper[2] = {p.pad_x - (p.kw - 1) * p.dil_x, p.pad_y - (p.kh - 1) * p.dil_y};
-        // the box of base pixels must produce exactly Q x P positions per image
-        const int q_tm = (p.in.x + upper[0] - lower[0] - 1) / p.stride_x + 1, p_tm = (p.in.y + upper[1] - lower[1] - 1) / p.stride_y + 1;
-        if (q_tm != P.Q || p_tm != P.P) return fail(CLDNN_B200_UNSUPPORTED_SIZE, "conv_featrows: im2col traversal does not match the output size");
-        cuuint32_t step[4] = {1, (cuuint32_t)p.stride_x, (cuuint32_t)p.stride_y, 1};
-        cr = fr_encode_im2col(&P.tmX, dt, 4, in_ptr, dims, strides, lower, upper, bke, (cuuint32_t)P.cols, step, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else {
-        const int sx = p.stride_x, sy = p.stride_y;                  // a pointwise strided convolution reads a strided view of the input
-        const bool view = sx != 1 || sy != 1;
-        cuuint64_t dims[4] = {(cuuint64_t)p.in.px, (cuuint64_t)(view ? P.Q : p.in.x), (cuuint64_t)(view ? P.P : p.in.y), (cuuint64_t)p.in.b};
-        cuuint64_t strides[3] = {(cuuint64_t)(xs * sx), (cuuint64_t)(p.in.py * sy * es), (cuuint64_t)(p.in.pb * es)};
-        cuuint32_t box[4] = {bke, (cuuint32_t)pl.bw, (cuuint32_t)pl.bh, (cuuint32_t)pl.bb}; cuuint32_t one[4] = {1, 1, 1, 1};
-        cr = fr_encode_tiled(&P.tmX, dt, 4, in_ptr, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-    if (cr != CUDA_SUCCESS) return fail(CLDNN_B200_DEVICE_ERROR, "conv_featrows: activation tensor map rejected by the driver (CUresult " + std::to_string((int)cr) + ")");
+    auto encode_x = [&](CUtensorMap* tm, cuuint64_t features) -> int32_t {      // `features`: where the pixels' reduction ends
+        if (pl.mode == FR_FLAT) {
+            cuuint64_t dims[2] = {features, (cuuint64_t)P.M_total}; cuuint64_t strides[1] = {(cuuint64_t)xs};
+            cuuint32_t box[2] = {bke, (cuuint32_t)P.cols}; cuuint32_t one[2] = {1, 1};
+            cr = fr_encode_tiled(tm, dt, 2, in_ptr, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        } else if (pl.mode == FR_IM2COL) {
+            cuuint64_t dims[4] = {features, (cuuint64_t)p.in.x, (cuuint64_t)p.in.y, (cuuint64_t)p.in.b};
+            cuuint64_t strides[3] = {(cuuint64_t)xs, (cuuint64_t)(p.in.py * es), (cuuint64_t)(p.in.pb * es)};
+            int lower[2] = {-p.pad_x, -p.pad_y};
+            int upper[2] = {p.pad_x - (p.kw - 1) * p.dil_x, p.pad_y - (p.kh - 1) * p.dil_y};
+            // the box of base pixels must produce exactly Q x P positions per image
+            const int q_tm = (p.in.x + upper[0] - lower[0] - 1) / p.stride_x + 1, p_tm = (p.in.y + upper[1] - lower[1] - 1) / p.stride_y + 1;
+            if (q_tm != P.Q || p_tm != P.P) return fail(CLDNN_B200_UNSUPPORTED_SIZE, "conv_featrows: im2col traversal does not match the output size");
+            cuuint32_t step[4] = {1, (cuuint32_t)p.stride_x, (cuuint32_t)p.stride_y, 1};
+            cr = fr_encode_im2col(tm, dt, 4, in_ptr, dims, strides, lower, upper, bke, (cuuint32_t)P.cols, step, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        } else {
+            const int sx = p.stride_x, sy = p.stride_y;                  // a pointwise strided convolution reads a strided view of the input
+            const bool view = sx != 1 || sy != 1;
+            cuuint64_t dims[4] = {features, (cuuint64_t)(view ? P.Q : p.in.x), (cuuint64_t)(view ? P.P : p.in.y), (cuuint64_t)p.in.b};
+            cuuint64_t strides[3] = {(cuuint64_t)(xs * sx), (cuuint64_t)(p.in.py * sy * es), (cuuint64_t)(p.in.pb * es)};
+            cuuint32_t box[4] = {bke, (cuuint32_t)pl.bw, (cuuint32_t)pl.bh, (cuuint32_t)pl.bb}; cuuint32_t one[4] = {1, 1, 1, 1};
+            cr = fr_encode_tiled(tm, dt, 4, in_ptr, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        }
+        if (cr != CUDA_SUCCESS) return fail(CLDNN_B200_DEVICE_ERROR, "conv_featrows: activation tensor map rejected by the driver (CUresult " + std::to_string((int)cr) + ")");
+        return CLDNN_B200_SUCCESS;
+    };
+    for (int g = 0; g < (P.group_maps ? p.groups : 1); ++g)
+        if (const int32_t st = encode_x(&P.tmX[g], (cuuint64_t)(P.group_maps ? (g + 1) * p.ifm : p.in.px))) return st;
     {
         cuuint64_t dims[3] = {(cuuint64_t)p.w_px, (cuuint64_t)(p.kh * p.kw), (cuuint64_t)p.ofm};
         cuuint64_t strides[2] = {(cuuint64_t)(p.w_px * es), (cuuint64_t)(p.w_po * es)};

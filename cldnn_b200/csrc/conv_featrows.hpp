@@ -8,8 +8,13 @@ namespace b200 {
 
 // A convolution in groups as the tensor-core kernels see it: every feature tile of 128 lies inside one group and reads that group's
 // slice of the input features (a channel offset of the activation copies), with weights that hold the group's features only, zero
-// padded to whole chunks of the reduction.  A chunk that reaches past the slice meets the padding's zeros.  `p` comes in with feature
-// counts per group and leaves with all output features in `ofm`; `ifm` stays the reduction's.
+// padded to whole chunks of the reduction.  A chunk that reaches past the slice meets the padding's zeros, which is enough for integers;
+// in fp16 zero times an Inf or NaN of the next group would be NaN, so there each group gets a tensor map that ends with its slice (zeros
+// come in behind it), for up to kGroupMaps groups.  `p` comes in with feature counts per group and leaves with all output features in
+// `ofm`; `ifm` stays the reduction's.
+constexpr int kGroupMaps = 4;
+inline int64_t chunk_bytes(int64_t cs) { return cs % 128 == 0 ? 128 : (cs % 64 == 0 ? 64 : 32); }   // of a tap's `cs` stored bytes
+inline bool slices_overhang(const cldnn_b200_conv_params& p) { return p.groups > 1 && p.in.dtype == CLDNN_B200_F16 && p.ifm * 2 % chunk_bytes(p.w_px * 2); }
 inline bool grouped_view(cldnn_b200_conv_params& p, std::string* why)
 {
     auto no = [&](const char* m) { if (why) *why = m; return false; };
@@ -18,6 +23,7 @@ inline bool grouped_view(cldnn_b200_conv_params& p, std::string* why)
     if (p.groups < 1 || p.fused_eltw) return no("grouped convolution: no fused residual");
     if (p.ofm < 128 || p.ofm % 128 || p.ifm * es % 16) return no("grouped convolution: whole feature tiles of 128 and 16-byte slices per group");
     if (p.w_px * es % 32 || p.w_px < p.ifm || p.w_px * es >= p.ifm * es + 128) return no("grouped convolution: weights must hold one group's features, padded to whole chunks");
+    if (p.groups > kGroupMaps && slices_overhang(p)) return no("grouped fp16 convolution: slices of more than four groups must be whole chunks of the reduction");
     p.ofm *= p.groups;
     return true;
 }
