@@ -12,7 +12,7 @@ input in L2); `e2e` includes, every step, the copy of a fresh batch from pinned 
 class probabilities.  The timed region of K steps is repeated until at least --min-seconds have been measured; the line
 reports the median repeat (and the fastest and slowest).  After the timed regions, outside them, rank 0 checks the very
 network it timed against the CPU oracle on the first images of a batch (`parity`) and times every primitive on a
-profiling engine (`per_primitive`, `roofline`).
+profiling engine (`roofline`; the rows themselves go to stderr as `per_primitive`, and with --table to a file).
 """
 import argparse
 import json
@@ -640,7 +640,8 @@ def main():
         line["parity"] = parity
         if cpu is not None and world == 1:
             line["cpu_baseline"] = cpu
-        line["per_primitive"] = table
+        # one short line on stdout (a reader of its tail gets all of it); the rows behind the roofline go to stderr
+        print(json.dumps({"per_primitive": table}), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     if world > 1:
         dist.destroy_process_group()
