@@ -130,3 +130,11 @@ def test_refused(plan, change):
         else:
             setattr(p.in_, k, v)
     assert plan(p, src_at, 1 << 24) is None
+
+
+@pytest.mark.parametrize("f,images,taken", [(1, 20, True), (1, 21, False), (2, 21, True)])
+def test_one_feature_of_many_pixels(plan, f, images, taken):
+    """A single feature out of a wide row stays with the general kernel from 2^18 pixels on."""
+    p = abi.ReorderParams()
+    p.in_, p.out = inner_slice(abi.U8, images, f, 112, 112, 32, 0), planar(abi.U8, images, f, 112, 112, 0, 0)
+    assert (plan(p, 1 << 20, 1 << 30) is not None) == taken
