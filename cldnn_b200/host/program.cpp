@@ -857,7 +857,7 @@ void network_impl::pick_kernel(node* n, const std::vector<std::string>& candidat
     set_tune(0);
     // the key carries the generation of the kernel set: timings taken on older kernels must not be reused.  `key_params`:
     // the constants with the fields that do not bear on the choice cleared (same size as `params`)
-    const std::string hash = fnv1a_hex(key_params ? key_params : params, psize, n->p.type + "#g3");
+    const std::string hash = fnv1a_hex(key_params ? key_params : params, psize, n->p.type + "#g4");
     if (opts.tuning != tuning_mode::tuning_disabled) {
         auto it = tuning_cache.find(hash);
         if (it != tuning_cache.end()) {
