@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <mutex>
 #include "conv_featrows.hpp"
+#include "conv_tile_cost.hpp"
 #include "conv_epilogue.cuh"
 
 namespace b200 {
@@ -385,16 +386,15 @@ bool fr_plan(const cldnn_b200_conv_params& p, int variant, FrPlan& pl, std::stri
 int fr_inner_product_variant(const cldnn_b200_conv_params& p)
 {
     if (p.groups != 1 || p.kh != 1 || p.kw != 1 || p.in.x != 1 || p.in.y != 1 || p.pad_x || p.pad_y || p.stride_x != 1 || p.stride_y != 1) return -1;
-    constexpr int64_t kSMs = 148;
     const int64_t cs = p.in.px * (p.in.dtype == CLDNN_B200_F16 ? 2 : 1), n = p.out.b, m_tiles = (p.ofm + kRows - 1) / kRows;
     const int64_t steps = cs / chunk_bytes(cs);
     int ci = 0;                                                      // kCols index: 16, 32, 64, 128
     auto n_tiles = [&](int i) { return (n + kCols[i] - 1) / kCols[i]; };
     auto widest = [&](int i) { int s = kFrSplits - 1; while (s > 0 && (int64_t)(n_tiles(i) > 1 ? 4 : 1) * (1 << s) > steps) --s; return s; };
     while (ci < 3 && kCols[ci] < n) ++ci;
-    while (ci > 1 && (m_tiles * n_tiles(ci) << widest(ci)) < kSMs) --ci;
+    while (ci > 1 && (m_tiles * n_tiles(ci) << widest(ci)) < kCostSMs) --ci;
     int si = widest(ci);
-    while (si > 0 && (m_tiles * n_tiles(ci) << si) > 2 * kSMs) --si;
+    while (si > 0 && (m_tiles * n_tiles(ci) << si) > 2 * kCostSMs) --si;
     return si > 0 ? ci * kFrSplits + si : -1;
 }
 
@@ -415,12 +415,12 @@ double fr_cost(const cldnn_b200_conv_params& p, int& variant)
     for (int v = 0; v < kFrVariants; ++v) {
         FrPlan pl;
         const int64_t cols = kCols[v / kFrSplits], split = 1 << (v % kFrSplits), ctas = m_tiles * ((pixels + cols - 1) / cols) * split;
-        const int64_t resident = (split == 8 ? 128 : (split == 4 ? 144 : 148)) * (cols == 256 ? 1 : 2);
+        const int64_t resident = (split == 8 ? 128 : (split == 4 ? 144 : kCostSMs)) * (cols == 256 ? 1 : 2);
         if (ctas > resident || !fr_plan(p, v, pl, nullptr, false)) continue;
         const double valid = (double)std::min(cols, pixels);
         const double main = (double)((steps + split - 1) / split) * (c.step + c.step_row * (double)(kRows + cols) * ((double)bk / 128.0));
         const double epi = c.col * (double)cols + c.gather * valid / (double)split + (split > 1 ? c.exchange_col * valid + c.exchange : 0.0);
-        const double t = c.launch + (main + epi) * (1.0 + c.share * std::max(0.0, (double)ctas / 148.0 - 1.0));
+        const double t = c.launch + (main + epi) * (1.0 + c.share * std::max(0.0, (double)ctas / (double)kCostSMs - 1.0));
         if (variant < 0 || t < best) { best = t; variant = v; }
     }
     return best;

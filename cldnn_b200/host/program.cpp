@@ -1053,7 +1053,7 @@ void network_impl::prepare_kernel(node* n)
             const int64_t kflat = cp.in.pb;
             cp.in.f = (int32_t)kflat; cp.in.x = cp.in.y = 1; cp.in.px = cp.in.py = kflat; cp.ifm = (int32_t)kflat;
         }
-        // a convolution in 2..4 groups runs as a dense one on block-diagonal weights (AlexNet's split layers)
+        // a convolution in 2..4 groups (AlexNet's split layers) runs group by group where the kernel takes it, else dense on block-diagonal weights
         const bool dense_groups = cp.groups >= 2 && cp.groups <= 4 && !fc;
         const bool try_tc = ((is_int8(in.data_type) && w.data_type == data_types::i8) || half_tc) && (cp.groups == 1 || dense_groups) && cp.in.pf == 1 && cp.in.px % 32 == 0 && cp.out.pf == 1;
         const char* tc_kernel = half_tc ? "conv_f16_tc" : "conv_i8_tc";

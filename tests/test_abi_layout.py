@@ -16,7 +16,7 @@ HEADER = os.path.join(ROOT, "include", "cldnn_b200.h")
 
 STRUCTS = {
     "cldnn_b200_tensor": abi.Tensor, "cldnn_b200_conv_params": abi.ConvParams, "cldnn_b200_args": abi.Args,
-    "cldnn_b200_pool_params": abi.PoolParams, "cldnn_b200_fc_params": abi.FcParams,
+    "cldnn_b200_pool_params": abi.PoolParams, "cldnn_b200_lrn_pool_params": abi.LrnPoolParams, "cldnn_b200_fc_params": abi.FcParams,
     "cldnn_b200_softmax_params": abi.SoftmaxParams, "cldnn_b200_eltwise_params": abi.EltwiseParams,
     "cldnn_b200_reorder_params": abi.ReorderParams, "cldnn_b200_lrn_params": abi.LrnParams,
     "cldnn_b200_activation_params": abi.ActivationParams, "cldnn_b200_engine_info": abi.EngineInfo,
@@ -28,6 +28,7 @@ def test_ctypes_mirror_matches_header_sizes():
     for name in STRUCTS:
         src += 'printf("%s %%zu\\n", sizeof(%s));\n' % (name, name)
     src += 'printf("tune_off %zu\\n", offsetof(cldnn_b200_conv_params, tune));\n'
+    src += 'printf("constant_off %zu\\n", offsetof(cldnn_b200_conv_params, constant_params));\n'
     src += 'printf("act_off %zu\\n", offsetof(cldnn_b200_conv_params, act));\nreturn 0;}\n'
     with tempfile.TemporaryDirectory() as d:
         c = os.path.join(d, "s.c")
@@ -38,6 +39,7 @@ def test_ctypes_mirror_matches_header_sizes():
     for name, cls in STRUCTS.items():
         assert sizes[name] == C.sizeof(cls), name
     assert sizes["tune_off"] == abi.ConvParams.tune.offset
+    assert sizes["constant_off"] == abi.ConvParams.constant_params.offset
     assert sizes["act_off"] == abi.ConvParams.act.offset
 
 
